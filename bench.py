@@ -268,8 +268,8 @@ FP32_TRAFFIC = {"w2z": "step_fp32_w2z", "w2q": "step_fp32_w2q", "w3": "step_fp32
 SCHEDULE_NOTES = {
     "fast": "two passes without divisions (rt_fast.cu): within 1e-12 relative L-inf of the reference per step, "
             "not bit-identical",
-    "split": "two passes, the reference's arithmetic bit for bit (rt_split.cu)",
-    "tma": "fused plane kernel, the reference's arithmetic bit for bit (rt_step3.cuh)",
+    "split": "two passes over slabs, the reference's arithmetic bit for bit (rt_exact.cu)",
+    "tma": "two passes over slabs, the reference's arithmetic bit for bit (rt_exact.cu)",
 }
 
 

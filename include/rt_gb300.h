@@ -176,9 +176,16 @@ int rt_diagnose(rt_handle* h, rt_budget* out, double* E_int, double* meanfl_int,
 int rt_get_tendency(rt_handle* h, double* dE, double* meanfl);
 
 /* Schedule of the step kernel.  variant:
- *   2  = plane tiled with bulk-copy (TMA) staging of the E planes (default;
- *        used when a plane of E is a multiple of 16 bytes)
- *   3  = the same with several z planes per work item (small x-y planes)
+ *   2  = the default.  binary64: the reference's arithmetic with its
+ *        divisions on the integer pipes, one launch for small fields and two
+ *        passes over slabs of the slowest axis for the others (the slab's
+ *        flux fields are allocated by the first such step: 48 bytes per cell
+ *        of a slab of about 2 M cells or one plane of the slowest axis; a
+ *        handle without room for them steps with the plane kernel).
+ *        binary32: plane tiled with bulk-copy (TMA) staging of the E planes,
+ *        used when a plane of E is a multiple of 16 bytes
+ *   3  = plane tiled with TMA staging, several z planes per work item (small
+ *        x-y planes)
  *   0  = plane tiled with plain loads,  1 = one thread per cell
  *   9  = binary32: persistent, warp-specialised, every operand staged
  *   13 = binary32: the same for small planes, z slices per work item
@@ -187,11 +194,10 @@ int rt_get_tendency(rt_handle* h, double* dE, double* meanfl);
  *   18 = 14 with the cell-pair arithmetic on packed f32x2 instructions and
  *        the next plane's operands prefetched into L2 (the production
  *        binary32 step)
- *   15 = binary64 in two passes: every face flux evaluated once into flux
- *        fields (allocated by this call: 48 bytes per cell plus the face-0
- *        planes), then divergence and update
- *   16 = binary64 fast: the two passes of 15 without divisions (limiter
- *        slope selected exactly, update regrouped; 8 more bytes per cell);
+ *   15 = binary64: as 2
+ *   16 = binary64 fast: two passes without divisions (limiter slope selected
+ *        exactly, update regrouped; its fields, 56 bytes per cell, are
+ *        allocated by this call);
  *        within a few units in the last place of the reference's result per
  *        step, NOT bit-identical to it.  band = m values per band of its
  *        spectral-plane order (1: natural order; a width that does not

@@ -51,7 +51,10 @@ struct rt_handle {
   double* force = nullptr;      // its interior 5D field (x,y,k,l,m)
   long long force_gen = 0;      // changes with every rt_set_forcing
   double dzt1 = 0.0;            // dzt(1), the bottom cell's spacing
-  SplitFluxes split{};          // flux fields of the two-pass binary64 step (allocated on selection)
+  SplitFluxes split{};          // flux fields of the fast binary64 step (allocated on selection)
+  SplitFluxes slab{};           // flux scratch of the bit-exact step's slabs (allocated by the first such step)
+  double* slab_mem = nullptr;
+  int slab_state = 0;           // 0: not asked for yet, 1: there, -1: no memory for it
   double* mu = nullptr;         // fast binary64 step: 1 - dt*lambda per cell (allocated on selection)
   double* tab64 = nullptr;      // and its tables dt/d_a (offsets toff[0..5])
   int uc_holds = 0;             // uc/ucl hold 0: uCFL of the bit-exact kernels, 1: h of the fast step
@@ -266,6 +269,31 @@ static bool fast_ready(const rt_handle* h) {
   return split && h->mu && h->tab64;
 }
 
+// scratch of the bit-exact step's slabs, one allocation; false when the
+// memory is not there (the handle then keeps the fused kernels, which need none)
+static bool slab_scratch(rt_handle* h) {
+  if (h->slab_state) return h->slab_state > 0;
+  long long len[7], total = 0;
+  for (int a = 0; a < 7; a++) {
+    len[a] = a < 6 ? exact_scratch(h->d, a) : exact_scratch_z0(h->d);
+    total += (len[a] + 1) / 2 * 2;
+  }
+  double* p = nullptr;
+  if (cudaMalloc((void**)&p, (size_t)total * sizeof(double)) != cudaSuccess) {
+    cudaGetLastError();
+    h->slab_state = -1;
+    return false;
+  }
+  h->bytes += total * (long long)sizeof(double);
+  h->slab_mem = p;
+  for (int a = 0; a < 7; a++) {
+    (a < 6 ? h->slab.f[a] : h->slab.f0[2]) = len[a] > 0 ? p : nullptr;
+    p += (len[a] + 1) / 2 * 2;
+  }
+  h->slab_state = 1;
+  return true;
+}
+
 // one step of the handle from buffer src into 1 - src; returns the kernels launched
 static cudaError_t step_once(rt_handle* h, int src, int* nlaunch) {
   if (h->p.precision == RT_FP64) {
@@ -279,13 +307,13 @@ static cudaError_t step_once(rt_handle* h, int src, int* nlaunch) {
     }
     cudaError_t e = ensure_uc(h, 0);
     if (e != cudaSuccess) return e;
-    // the two-pass step once its fields exist (rt_set_tuning allocates them;
-    // a field with no axis longer than one keeps the fused step)
-    bool split = false;
-    for (int a = 0; a < 6; a++) split = split || h->split.f[a] != nullptr;
-    if (h->tune.variant == RT_VARIANT_SPLIT && split) {
-      *nlaunch = 2;
-      return launch_step_split(make_step_args<double>(h, src), h->split, h->st);
+    // the bit-exact step of every variant that does not name one of the
+    // plane kernels (rt_exact.cu)
+    const int v = h->tune.variant;
+    if (v != RT_VARIANT_PLANE && v != RT_VARIANT_CELL && v != RT_VARIANT_GROUP && h->d.ncell < (1ll << 31)) {
+      *nlaunch = 1;
+      if (!exact_in_slabs(h->d)) return launch_step_exact_cells(make_step_args<double>(h, src), h->st);
+      if (slab_scratch(h)) return launch_step_exact_slabs(make_step_args<double>(h, src), h->slab, h->st, nlaunch);
     }
     *nlaunch = 1;
     return launch_step<double>(make_step_args<double>(h, src), h->tune, h->st);
@@ -294,7 +322,7 @@ static cudaError_t step_once(rt_handle* h, int src, int* nlaunch) {
   return launch_step<float>(make_step_args<float>(h, src), h->tune, h->st);
 }
 
-// flux fields of the two-pass binary64 step, for the axes with n > 1
+// flux fields of the fast binary64 step, for the axes with n > 1
 static int ensure_split(rt_handle* h) {
   const Dims& d = h->d;
   for (int a = 0; a < 6; a++) {
@@ -1088,6 +1116,7 @@ int rt_destroy(rt_handle* h) {
   cudaFree(h->seed);
   cudaFree(h->force);
   for (int a = 0; a < 6; a++) { cudaFree(h->split.f[a]); cudaFree(h->split.f0[a]); }
+  cudaFree(h->slab_mem);
   cudaFree(h->mu);
   cudaFree(h->tab64);
   for (auto& kv : h->timers) {
@@ -1629,10 +1658,6 @@ int rt_set_tuning(rt_handle* h, int variant, int band, int threads) {
   if (band < 1 || band > 1024) return fail(h, RT_ERR_ARG, "rt_set_tuning: band %d out of range", band);
   if (threads != 128 && threads != 256 && threads != 512 && threads != 1024)
     return fail(h, RT_ERR_ARG, "rt_set_tuning: threads must be 128, 256, 512 or 1024");
-  if (variant == RT_VARIANT_SPLIT && h->p.precision == RT_FP64) {
-    const int rc = ensure_split(h);
-    if (rc) return rc;
-  }
   if (variant == RT_VARIANT_FAST && h->p.precision == RT_FP64) {
     const int rc = ensure_fast(h);
     if (rc) return rc;

@@ -1,6 +1,6 @@
 // rt_fast.cu -- fast binary64 step (variant RT_VARIANT_FAST).
 //
-// The same two passes as the two-pass bit-exact step (rt_split.cu): every
+// The same two passes as the two-pass bit-exact step (rt_exact.cu): every
 // face flux is evaluated once into the binary64 flux fields, then a second
 // pass forms the divergence, the mean-flow term and the update.  What
 // changes is the arithmetic (rt_fast.cuh): no division and no binary64

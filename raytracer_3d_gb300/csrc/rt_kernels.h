@@ -72,7 +72,7 @@ cudaError_t launch_lam_combine(const double* lx, const double* ly, const double*
 #define RT_VARIANT_W2Z 14     // binary32: 2-wide blocks, z-march
 #define RT_VARIANT_W2Q 18     // the same with the cell-pair arithmetic on packed f32x2 instructions and
                               // the next plane's operands prefetched into L2 (the binary32 production step)
-#define RT_VARIANT_SPLIT 15   // binary64: every face flux once, two passes (rt_split.cu)
+#define RT_VARIANT_SPLIT 15   // binary64: every face flux once, two passes (rt_exact.cu)
 #define RT_VARIANT_FAST 16    // binary64: two passes without divisions (rt_fast.cu), within 1e-12 of the reference
 struct StepTuning {
   int variant = RT_VARIANT_TMA;
@@ -154,14 +154,20 @@ cudaError_t launch_batch_fused(const BatchFused& F, int grid, int ga, cudaStream
 // rt_persist.cu, rt_persist_w2.cu); done = false when the tuning
 // does not select one of them or the shape does not fit them
 cudaError_t launch_persist(const StepArgs<float>& A, const StepTuning& tn, cudaStream_t st, bool& done);
-// two-pass binary64 step (rt_split.cu): the face fluxes of every axis with
-// n > 1 into f[a] (cell shape, the cell's right face) and f0[a] (face-0
-// plane, the layout of vlo[a]), then divergence, mean-flow term and update
+// bit-exact binary64 step without binary64 divisions (rt_exact.cu).  Flux
+// fields of a two-pass step: f[a] (the cell's right face) and f0[a] (the
+// face-0 plane, the layout of vlo[a])
 struct SplitFluxes {
   double* f[6];
   double* f0[6];
 };
-cudaError_t launch_step_split(const StepArgs<double>& A, const SplitFluxes& F, cudaStream_t st);
+// fields of more cells take the two passes over slabs, the others one launch
+bool exact_in_slabs(const Dims& d);
+// doubles of the slab scratch: flux field of axis a, and the face-0 plane of z
+long long exact_scratch(const Dims& d, int a);
+long long exact_scratch_z0(const Dims& d);
+cudaError_t launch_step_exact_cells(const StepArgs<double>& A, cudaStream_t st);
+cudaError_t launch_step_exact_slabs(const StepArgs<double>& A, const SplitFluxes& F, cudaStream_t st, int* nlaunch);
 // fast binary64 step (rt_fast.cu): the flux fields of the two-pass step,
 // h = |v|/2*(1-|v dt/d|) per face (hr: right faces, hl: face-0 planes),
 // mu = 1 - dt*lambda per cell and the per-axis tables c[a] = dt/d_a on the

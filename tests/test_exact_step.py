@@ -1,0 +1,63 @@
+"""The bit-exact binary64 step without binary64 divisions: its integer
+quotient against the division instruction (host, and on the GPU), and its
+two forms against the one-thread-per-cell kernel, which the parity tests
+hold to the oracle, at the edges of their ranges."""
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+from harness import ROOT, configs
+
+SRC = os.path.join(ROOT, "tests", "native", "exact_div_check.cu")
+
+
+def _check(tmp_path, *args, flags=()):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc not found")
+    exe = str(tmp_path / "exact_div_check")
+    subprocess.run([nvcc, "-gencode", "arch=compute_103a,code=sm_103a", "-O2", "-std=c++17", *flags,
+                    "-I" + os.path.join(ROOT, "raytracer_3d_gb300", "csrc"), "-o", exe, SRC], check=True)
+    r = subprocess.run([exe, *args], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("ulp", ["0", "1u", "0xffffffffu"])
+def test_integer_quotient_on_the_host(tmp_path, ulp):
+    _check(tmp_path, flags=("-DRT_RECIP_HOST_ULP=" + ulp,))
+
+
+@pytest.mark.gpu
+def test_integer_quotient_on_the_gpu(tmp_path):
+    _check(tmp_path, "--device")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("walls", [True, False])
+@pytest.mark.parametrize("n", [
+    (4, 4, 4, 8, 8, 16), (4, 4, 4, 8, 8, 18),     # last field of one launch, first of two passes
+    (16, 16, 16, 8, 8, 18), (15, 7, 12, 10, 12, 16),   # slabs over m; the last one shorter
+    (16, 16, 64, 2, 140, 1),                      # over l, and several of them
+    (160, 128, 110, 1, 1, 1), (2100, 1100, 1, 1, 1, 1),   # over z (its own face-0 plane) and y
+])
+def test_forms_equal_the_cell_kernel(n, walls):
+    import __graft_entry__ as g
+    g.build()
+    rng = np.random.default_rng(5)
+    exp = configs.shear_mini(n=n, upper=walls, lower=walls)
+    exp.fixed = (1e-3, 0.0, 1e-2)     # wavenumbers of collapsed axes
+    got = []
+    E0 = rng.random(n) ** 4 * 1e-3
+    for variant in ("cell", "tma", "split"):
+        m = configs.build_model(exp, "fp64")
+        m.E[(slice(2, -2),) * 6] = E0
+        m.set_state()
+        m.set_tuning(variant, 8, 256)
+        m.integrate(3)
+        got.append(m.get_state()[(slice(2, -2),) * 6].copy())
+        m.close()
+    assert np.isfinite(got[0]).all()
+    assert np.array_equal(got[1], got[0]) and np.array_equal(got[2], got[0])
