@@ -230,6 +230,14 @@ static StepArgs<T> make_step_args(const rt_handle* h, int src) {
   return A;
 }
 
+template <class T>
+static CoeffOut<T> coeff_out(rt_handle* h) {
+  CoeffOut<T> o;
+  for (int a = 0; a < 6; a++) { o.vel[a] = (T*)h->vel[a]; o.vlo[a] = (T*)h->vlo[a]; }
+  for (int c = 0; c < 3; c++) o.lam[c] = (T*)h->lam[c];
+  return o;
+}
+
 // set_forcing on the state about to be stepped (main.f90:69)
 static cudaError_t apply_forcing(rt_handle* h, int buf, cudaStream_t st) {
   const double dzt1 = h->dzt1;
@@ -1087,7 +1095,7 @@ int rt_create(const rt_dims* dims, const rt_params* params, rt_handle** out) {
       if ((rc = dev_alloc(h, (void**)&h->ucl[a], (size_t)(d.ncell / d.n[a]) * 8))) return bail(rc);
     }
   const DiagSizes ds = diag_sizes(d);
-  h->scratch_len = std::max(ds.scratch_doubles(), max_rate_partials(d)) + 8;
+  h->scratch_len = ds.scratch_doubles() + 8;
   if ((rc = dev_alloc(h, (void**)&h->scratch, h->scratch_len * sizeof(double)))) return bail(rc);
   if ((rc = dev_alloc(h, (void**)&h->vol3, 8 * d.nvol3 * sizeof(double)))) return bail(rc);
   if ((rc = dev_alloc(h, (void**)&h->result, 32 * sizeof(double)))) return bail(rc);
@@ -1193,67 +1201,28 @@ int rt_calc_parameter(rt_handle* h) {
   Phys ph{h->p.f0, h->p.sign_of_omega_i, h->p.dt};
   const Grid g = make_grid(h);
 
-  CoeffOut64 o64{};
-  std::vector<void*> tmp;
-  const bool fp64 = h->p.precision == RT_FP64;
-  int rc;
-  // binary64 destinations: the handle's own fields (FP64) or temporaries
-  for (int a = 0; a < 6; a++) {
-    if (fp64) {
-      o64.vel[a] = (double*)h->vel[a];
-      o64.vlo[a] = (double*)h->vlo[a];
-    } else {
-      void* p1 = nullptr; void* p2 = nullptr;
-      if ((rc = tmp_alloc(h, &p1, d.ncell * sizeof(double)))) goto cleanup;
-      tmp.push_back(p1);
-      if ((rc = tmp_alloc(h, &p2, (d.ncell / d.n[a]) * sizeof(double)))) goto cleanup;
-      tmp.push_back(p2);
-      o64.vel[a] = (double*)p1;
-      o64.vlo[a] = (double*)p2;
-    }
+  // scratch of the dispersion relation: a ring of m planes, 256 MB or the
+  // three planes it cannot do without
+  double* scratch = nullptr;
+  int ring = coeff_ring(d, 256ll << 20);
+  int rc = tmp_alloc(h, (void**)&scratch, (size_t)coeff_scratch(d, ring) * sizeof(double));
+  if (rc && ring > 3) {
+    ring = 3;
+    rc = tmp_alloc(h, (void**)&scratch, (size_t)coeff_scratch(d, ring) * sizeof(double));
   }
-  for (int c = 0; c < 3; c++) {
-    if (fp64) {
-      o64.lam[c] = (double*)h->lam[c];
-    } else {
-      void* p1 = nullptr;
-      if ((rc = tmp_alloc(h, &p1, d.ncell * sizeof(double)))) goto cleanup;
-      tmp.push_back(p1);
-      o64.lam[c] = (double*)p1;
-    }
-  }
-  {
-    cudaError_t e = launch_coeff(d, bg, g, ph, o64, h->st);
-    h->launches += 7;
-    if (e != cudaSuccess) { rc = fail(h, RT_ERR_CUDA, "coefficients: %s", cudaGetErrorString(e)); goto cleanup; }
-    ConstCoeff64 cf;
-    for (int a = 0; a < 6; a++) { cf.vel[a] = o64.vel[a]; cf.vlo[a] = o64.vlo[a]; }
-    e = launch_max_rate(d, g, cf, h->scratch, h->result, h->st);
-    h->launches += 2;
-    if (e != cudaSuccess) { rc = fail(h, RT_ERR_CUDA, "max rate: %s", cudaGetErrorString(e)); goto cleanup; }
-    if (!fp64) {
-      for (int a = 0; a < 6; a++) {
-        if ((e = launch_to_fp32(o64.vel[a], (float*)h->vel[a], d.ncell, h->st)) != cudaSuccess) break;
-        if ((e = launch_to_fp32(o64.vlo[a], (float*)h->vlo[a], d.ncell / d.n[a], h->st)) != cudaSuccess) break;
-        h->launches += 2;
-      }
-      if (e == cudaSuccess)
-        e = launch_lam_combine(o64.lam[0], o64.lam[1], o64.lam[2], d.n[0] > 1, d.n[1] > 1,
-                               d.n[2] > 1, (float*)h->lam[0], d.ncell, h->st);
-      h->launches += 1;
-      if (e != cudaSuccess) { rc = fail(h, RT_ERR_CUDA, "fp32 conversion: %s", cudaGetErrorString(e)); goto cleanup; }
-    }
-    e = cudaMemcpyAsync(&h->rate, h->result, sizeof(double), cudaMemcpyDeviceToHost, h->st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
-    if (e != cudaSuccess) { rc = fail(h, RT_ERR_CUDA, "calc_parameter: %s", cudaGetErrorString(e)); goto cleanup; }
-  }
+  if (rc) return rc;
+  int nl = 0;
+  cudaError_t e = h->p.precision == RT_FP64
+                      ? launch_coeff(d, bg, g, ph, coeff_out<double>(h), scratch, ring, h->result, &nl, h->st)
+                      : launch_coeff(d, bg, g, ph, coeff_out<float>(h), scratch, ring, h->result, &nl, h->st);
+  h->launches += nl;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&h->rate, h->result, sizeof(double), cudaMemcpyDeviceToHost, h->st);
+  cudaFreeAsync(scratch, h->st);   // stream-ordered: after the kernels
+  const cudaError_t e2 = cudaStreamSynchronize(h->st);
+  if (e == cudaSuccess) e = e2;
+  if (e != cudaSuccess) return fail(h, RT_ERR_CUDA, "coefficients: %s", cudaGetErrorString(e));
   h->have_coeff = true;
-  rc = refresh_ucfl(h);
-cleanup:
-  // stream-ordered frees run after the kernels that read the temporaries
-  for (void* p : tmp) { cudaFreeAsync(p, h->st); }
-  cudaStreamSynchronize(h->st);
-  return rc;
+  return refresh_ucfl(h);
 }
 
 int rt_max_rate(rt_handle* h, double* rate) {

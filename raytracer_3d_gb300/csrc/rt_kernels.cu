@@ -1,10 +1,9 @@
 // rt_kernels.cu -- sm_103a kernels of the time-stepping path:
-//   coefficient kernels   calc_parameter.f90:13-261
+//   cached uCFL           superbee_fluxes.f90:19
 //   fused step kernel     superbee_fluxes.f90 + integrate.f90:102-268
 //   budget kernels        diagnose.f90:46-329 (reductions)
 #include "rt_kernels.h"
 
-#include "rt_coeff.cuh"
 #include "rt_step.cuh"
 #include "rt_step2.cuh"
 #include "rt_step3.cuh"
@@ -24,116 +23,6 @@ __device__ __forceinline__ void decode(const Dims& d, long long v3, long long sp
   r = sp / d.n[3];
   c[4] = (int)(r % d.n[4]);
   c[5] = (int)(r / d.n[4]);
-}
-
-// ---------------------------------------------------------------------------
-// coefficients
-// ---------------------------------------------------------------------------
-// One thread per interior cell: the six right-face velocities and the three
-// growth rates, binary64.
-__global__ void __launch_bounds__(128) coeff_cells_kernel(Dims d, Background bg, Grid g, Phys ph,
-                                                          CoeffOut64 out) {
-  const long long v3 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v3 >= d.nvol3) return;
-  for (long long sp = blockIdx.y; sp < d.nspec; sp += gridDim.y) {
-    int c0[6];
-    decode(d, v3, sp, c0);
-    int c[6];
-#pragma unroll
-    for (int b = 0; b < 6; b++) c[b] = c0[b] + 1;  // Fortran indices
-    const long long p = v3 + sp * d.nvol3;
-    double v[6];
-    for (int a = 0; a < 6; a++) {
-      v[a] = face_velocity(d, bg, g, ph, a, c);
-      out.vel[a][p] = v[a];
-    }
-    double lx, ly, lz;
-    growth_rates(bg, g, ph, c, v[0], v[1], v[2], lx, ly, lz);
-    out.lam[0][p] = lx;
-    out.lam[1][p] = ly;
-    out.lam[2][p] = lz;
-  }
-}
-
-// One thread per cell of the face-0 plane of axis a.
-__global__ void __launch_bounds__(128) coeff_planes_kernel(Dims d, Background bg, Grid g, Phys ph,
-                                                           int a, double* out) {
-  long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long nplane = d.ncell / d.n[a];
-  if (q >= nplane) return;
-  int c[6];
-  long long r = q;
-  for (int b = 0; b < 6; b++) {
-    if (b == a) { c[b] = 0; continue; }
-    c[b] = (int)(r % d.n[b]) + 1;
-    r /= d.n[b];
-  }
-  out[q] = face_velocity(d, bg, g, ph, a, c);
-}
-
-// max over interior cells of sum_a max(|v_a(F-1)|,|v_a(F)|)/d_a(F): the
-// CFL rate that defines dt for the CFL-specified workloads.
-__global__ void __launch_bounds__(256) max_rate_kernel(Dims d, Grid g, ConstCoeff64 cf,
-                                                       double* partial) {
-  __shared__ double red[256];
-  const long long v3 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  double best = 0.0;
-  if (v3 < d.nvol3) {
-    for (long long sp = blockIdx.y; sp < d.nspec; sp += gridDim.y) {
-      int c[6];
-      decode(d, v3, sp, c);
-      const long long p = v3 + sp * d.nvol3;
-      double r = 0.0;
-      for (int a = 0; a < 6; a++) {
-        if (d.n[a] <= 1) continue;
-        const double vr = cf.vel[a][p];
-        const double vl = c[a] > 0 ? cf.vel[a][p - d.s[a]] : cf.vlo[a][plane_index(d, a, c)];
-        r = dadd(r, ddiv(fmax2(fabs(vl), fabs(vr)), g.d[a][pidx(c[a] + 1)]));
-      }
-      best = fmax2(best, r);
-    }
-  }
-  red[threadIdx.x] = best;
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] = fmax2(red[threadIdx.x], red[threadIdx.x + w]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) partial[blockIdx.y * gridDim.x + blockIdx.x] = red[0];
-}
-
-__global__ void max_reduce_kernel(const double* partial, long long n, double* out) {
-  __shared__ double red[256];
-  double best = 0.0;
-  for (long long i = threadIdx.x; i < n; i += blockDim.x) best = fmax2(best, partial[i]);
-  red[threadIdx.x] = best;
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] = fmax2(red[threadIdx.x], red[threadIdx.x + w]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[0] = red[0];
-}
-
-// binary64 -> binary32 copy of the coefficient fields; the binary32 form
-// keeps one combined growth rate lam = lambda_x[nx>1] + lambda_y[ny>1] +
-// lambda_z[nz>1], summed in binary64 before rounding.
-__global__ void to_fp32_kernel(const double* src, float* dst, long long n) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    dst[i] = __double2float_rn(src[i]);
-}
-
-__global__ void lam_combine_kernel(const double* lx, const double* ly, const double* lz, int ux,
-                                   int uy, int uz, float* dst, long long n) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    double s = 0.0;
-    if (ux) s += lx[i];
-    if (uy) s += ly[i];
-    if (uz) s += lz[i];
-    dst[i] = __double2float_rn(s);
-  }
 }
 
 // uCFL = |v*dt/d(f)| of every face of axis a (binary64 form), in the order of
@@ -484,35 +373,6 @@ static dim3 cell_grid(const Dims& d, int threads) {
   return dim3((unsigned)bx, (unsigned)by, 1);
 }
 
-cudaError_t launch_coeff(const Dims& d, const Background& bg, const Grid& g, const Phys& ph,
-                         const CoeffOut64& out, cudaStream_t st) {
-  coeff_cells_kernel<<<cell_grid(d, 128), 128, 0, st>>>(d, bg, g, ph, out);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  for (int a = 0; a < 6; a++) {
-    const long long nplane = d.ncell / d.n[a];
-    coeff_planes_kernel<<<(unsigned)((nplane + 127) / 128), 128, 0, st>>>(d, bg, g, ph, a, out.vlo[a]);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
-}
-
-long long max_rate_partials(const Dims& d) {
-  dim3 gr = cell_grid(d, 256);
-  return (long long)gr.x * gr.y;
-}
-
-cudaError_t launch_max_rate(const Dims& d, const Grid& g, const ConstCoeff64& cf, double* partial,
-                            double* out, cudaStream_t st) {
-  dim3 gr = cell_grid(d, 256);
-  max_rate_kernel<<<gr, 256, 0, st>>>(d, g, cf, partial);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  max_reduce_kernel<<<1, 256, 0, st>>>(partial, (long long)gr.x * gr.y, out);
-  return cudaGetLastError();
-}
-
 // ---- padded host array <-> unpadded device field, read / written by the GPU
 // through the host's page tables (devices with pageable memory access) ----
 // A warp moves one x row: row r of the interior is (y, z, k, l, m) in x-fastest
@@ -558,17 +418,6 @@ template cudaError_t launch_host_gather<double>(const double*, double*, const Di
 template cudaError_t launch_host_gather<float>(const double*, float*, const Dims&, cudaStream_t);
 template cudaError_t launch_host_scatter<double>(const double*, double*, const Dims&, cudaStream_t);
 template cudaError_t launch_host_scatter<float>(const float*, double*, const Dims&, cudaStream_t);
-
-cudaError_t launch_to_fp32(const double* src, float* dst, long long n, cudaStream_t st) {
-  to_fp32_kernel<<<4 * 152, 256, 0, st>>>(src, dst, n);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_lam_combine(const double* lx, const double* ly, const double* lz, int ux, int uy,
-                               int uz, float* dst, long long n, cudaStream_t st) {
-  lam_combine_kernel<<<4 * 152, 256, 0, st>>>(lx, ly, lz, ux, uy, uz, dst, n);
-  return cudaGetLastError();
-}
 
 PlaneSched make_sched(const Dims& d, const StepTuning& tn, int gz) {
   PlaneSched S;

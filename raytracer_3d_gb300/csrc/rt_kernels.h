@@ -19,15 +19,14 @@ template <class T> struct StepArgs;
 // bfl_xs, bfl_xe, bfl_ys, bfl_ye, ..., bfl_ms, bfl_me
 #define DIAG_RESULT_NV (DIAG_CELL_NV + 12)
 
-struct CoeffOut64 {
-  double* vel[6];
-  double* vlo[6];
-  double* lam[3];
-};
-
-struct ConstCoeff64 {
-  const double* vel[6];
-  const double* vlo[6];
+// destinations of the coefficient kernel: velocities, face-0 planes and
+// growth rates (binary64: x, y, z; binary32: lam[0], their sum over the axes
+// with n > 1)
+template <class T>
+struct CoeffOut {
+  T* vel[6];
+  T* vlo[6];
+  T* lam[3];
 };
 
 struct DiagSizes {
@@ -39,12 +38,14 @@ struct DiagSizes {
 // grid spacing of 0-based cell c along axis a
 __host__ __device__ __forceinline__ double g_d(const Grid& g, int a, int c) { return g.d[a][pidx(c + 1)]; }
 
-cudaError_t launch_coeff(const Dims& d, const Background& bg, const Grid& g, const Phys& ph,
-                         const CoeffOut64& out, cudaStream_t st);
-long long max_rate_partials(const Dims& d);
-cudaError_t launch_max_rate(const Dims& d, const Grid& g, const ConstCoeff64& cf, double* partial,
-                            double* out, cudaStream_t st);
-cudaError_t launch_to_fp32(const double* src, float* dst, long long n, cudaStream_t st);
+// coefficients (rt_coeff.cu): m planes of the scratch ring within `bytes`,
+// its length in doubles, and the launches; *rate (device) receives the CFL
+// rate, max over cells of sum_a max(|v_a(F-1)|,|v_a(F)|)/d_a(F)
+int coeff_ring(const Dims& d, long long bytes);
+long long coeff_scratch(const Dims& d, int ring);
+template <class T>
+cudaError_t launch_coeff(const Dims& d, const Background& bg, const Grid& g, const Phys& ph, const CoeffOut<T>& out,
+                         double* scratch, int ring, double* rate, int* nlaunch, cudaStream_t st);
 // padded host array (pageable, read / written by the GPU directly) <-> the
 // unpadded device field
 template <class T>
@@ -54,8 +55,6 @@ cudaError_t launch_host_scatter(const T* src, double* host, const Dims& d, cudaS
 cudaError_t launch_ucfl(const Dims& d, const Grid& g, double dt, const double* const* vel,
                         const double* const* vlo, double* const* uc, double* const* ucl,
                         cudaStream_t st);
-cudaError_t launch_lam_combine(const double* lx, const double* ly, const double* lz, int ux, int uy,
-                               int uz, float* dst, long long n, cudaStream_t st);
 // step kernel variants (numbers are the rt_set_tuning codes): the
 // plane-tiled kernel (rt_step2.cuh), the one-thread-per-cell kernel
 // (rt_step.cuh), kept as the fallback for planes that do not fit in shared
