@@ -506,7 +506,7 @@ def bench_serving(nreq=60, rate=20.0, seed=77, budget=120e9, baseline_req=12, st
     from raytracer_3d_gb300.serve import GpuExecutor, SequentialExecutor, Server, poisson_requests
 
     def serve(reqs):
-        ex = GpuExecutor("fp32", batch_tuning=(8, 512, 1, 16), persistent=512)
+        ex = GpuExecutor("fp32", batch_tuning=(8, 512, 1, 16))
         rep = Server(ex, budget_bytes=budget, chunk_max=50, setup_workers=8).run(reqs)
         ex.close()
         breakdown = {k: round(v, 2) for k, v in ex.times.items()}

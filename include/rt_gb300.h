@@ -182,8 +182,9 @@ int rt_get_tendency(rt_handle* h, double* dE, double* meanfl);
  *        flux fields are allocated by the first such step: 48 bytes per cell
  *        of a slab of about 2 M cells or one plane of the slowest axis; a
  *        handle without room for them steps with the plane kernel).
- *        binary32: plane tiled with bulk-copy (TMA) staging of the E planes,
- *        used when a plane of E is a multiple of 16 bytes
+ *        binary32: threads marching along k, the next k's operands copied
+ *        ahead into shared memory; fields above 2^30 cells: plane tiled with
+ *        bulk-copy (TMA) staging of the E planes
  *   3  = plane tiled with TMA staging, several z planes per work item (small
  *        x-y planes)
  *   0  = plane tiled with plain loads,  1 = one thread per cell
@@ -191,9 +192,9 @@ int rt_get_tendency(rt_handle* h, double* dE, double* meanfl);
  *   13 = binary32: the same for small planes, z slices per work item
  *   14 = binary32: persistent, warp-specialised, 2-wide cell blocks, CTAs
  *        marching along z
- *   18 = 14 with the cell-pair arithmetic on packed f32x2 instructions and
- *        the next plane's operands prefetched into L2 (the production
- *        binary32 step)
+ *   18 = as 2; fields above 2^30 cells: 14 with the cell-pair arithmetic on
+ *        packed f32x2 instructions and the next plane's operands prefetched
+ *        into L2
  *   15 = binary64: as 2
  *   16 = binary64 fast: two passes without divisions (limiter slope selected
  *        exactly, update regrouped; its fields, 56 bytes per cell, are
@@ -269,13 +270,14 @@ const char* rt_batch_last_error(const rt_batch* b);
 /* band, CTA size (128/256/512/1024), sweep order (0/1) and steps per captured
  * graph (even); chosen by the autotuner (raytracer_3d_gb300.autotune) */
 int rt_batch_set_tuning(rt_batch* b, int band, int threads, int sweep, int graph_steps);
-/* binary32 members whose x-y planes fill a CTA of `threads` consumer
+/* 0 (default): every member is stepped by one kernel; binary32: threads
+ * marching along k, any extents, one launch for up to 80 members.  Otherwise
+ * binary32 members whose x-y planes fill a CTA of `threads` consumer
  * threads (128/256/512; x and y extents multiples of 4) are stepped by the
  * batched warp-specialised kernel with every operand staged by bulk copies;
  * members with smaller planes (every axis z..m longer than one) by its form
  * with several z slices per work item (256 or 512 consumer threads); the
- * others by the z-group / plane kernels.  0 puts every member in the last
- * class.  Default 256.  No effect on results. */
+ * rest as with 0.  No effect on results. */
 int rt_batch_set_persistent(rt_batch* b, int threads);
 /* consumer threads (256 or 512) of the small-plane class alone; 0 turns
  * that class off, -1 (default) follows rt_batch_set_persistent */

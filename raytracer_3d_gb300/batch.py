@@ -26,7 +26,7 @@ class Batch:
         for m in self.models:
             m._state_on_device = True
         self.tuning = (8, 256, 0, 16)
-        self.persistent = 256
+        self.persistent = 0
         self.slices = -1
         self.fused = False
 
@@ -39,7 +39,8 @@ class Batch:
         self.tuning = (band, threads, sweep, graph_steps)
 
     def set_persistent(self, threads=256):
-        """consumer threads of the warp-specialised class (0: off)"""
+        """consumer threads of the warp-specialised class (0, as in a new
+        batch: off)"""
         self._check(self._lib.rt_batch_set_persistent(self._b, int(threads)), "rt_batch_set_persistent")
         self.persistent = int(threads)
 

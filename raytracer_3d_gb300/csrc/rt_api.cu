@@ -405,6 +405,8 @@ struct rt_batch {
   size_t smem = 0;
   bool tma = false;
   bool group = false;           // z-group items (rt_step4.cuh)
+  std::vector<StepArgs<float>> march[2];  // binary32: the class's arguments for the two parities (rt_march.cu);
+                                          // empty where a member is too large for it
   long long max_nxy = 0;
   StepTuning tune;
   int grid = 0;
@@ -416,9 +418,9 @@ struct rt_batch {
   cudaEvent_t ev = nullptr;
   std::string err;
   // members stepped by the batched fully staged kernel (binary32 form, planes
-  // that fill a CTA of pthreads consumer threads); the others use the arrays
-  // above (nq members)
-  int pthreads = 256;           // 0: every member in the other class
+  // that fill a CTA of pthreads consumer threads, on request); the others use
+  // the arrays above (nq members)
+  int pthreads = 0;             // 0: every member in the other class
   int np = 0, nq = 0;
   void* d_pmem[2] = {nullptr, nullptr};
   long long* d_pfirst = nullptr;
@@ -464,7 +466,8 @@ static void batch_free_graphs(rt_batch* b) {
 // kernel launches per batch step
 static int batch_kernels(const rt_batch* b) {
   const int persistent = b->fgrid > 0 ? 1 : (b->np > 0 ? 1 : 0) + (b->ns6 > 0 ? 1 : 0);
-  return (int)b->forced.size() + persistent + (b->nq > 0 ? 1 : 0);
+  const int rest = b->nq == 0 ? 0 : (b->march[0].empty() ? 1 : march_batch_launches(b->nq));
+  return (int)b->forced.size() + persistent + rest;
 }
 
 static BatchFused batch_fused_args(const rt_batch* b, int par) {
@@ -566,6 +569,8 @@ static cudaError_t batch_launch(rt_batch* b, int par, bool force = true) {
       e = launch_batch_w6(b->d_smem6[par], b->d_sfirst, b->ns6, b->sthreads, b->sns, b->sstage, b->sgrid, b->st);
   }
   if (e != cudaSuccess || !b->nq) return e;
+  if (!b->march[par].empty())
+    return launch_march_batch(b->march[par].data(), b->nq, b->tune.band, b->tune.sweep, b->st);
   const void* mem = b->d_mem[par];
   const int n = b->nq;
   if (b->group) return launch_batch_group<T>(mem, b->d_first, n, b->smem, b->tune.threads, b->grid, b->st);
@@ -706,6 +711,17 @@ static int batch_build(rt_batch* b) {
   batch_plan_fused(b);
   const int n = (int)qm.size();
   b->nq = n;
+  bool march = sizeof(T) == 4 && n > 0;
+  for (int j : qm) march = march && march_ok(b->mem[j]->d);
+  for (int par = 0; par < 2; par++) {
+    b->march[par].clear();
+    if (march)
+      for (int j : qm) {
+        rt_handle* h = b->mem[j];
+        b->march[par].push_back(make_step_args<float>(h, par == 0 ? h->cur : 1 - h->cur));
+        b->cur0[j] = h->cur;
+      }
+  }
   std::vector<BatchMember<T>> arr[2];
   std::vector<long long> first(n + 1, 0);
   size_t smem = 0;
@@ -724,8 +740,8 @@ static int batch_build(rt_batch* b) {
   // the TMA plane kernel covers the largest plane with at most RT_TMA_MAXC cells per thread
   if ((b->max_nxy + b->tune.threads - 1) / b->tune.threads > RT_TMA_MAXC) tma = false;
   // the plain-load batch kernel has no 1024-thread form
-  if (!tma && !group && b->tune.threads > 512) b->tune.threads = 512;
-  for (int i = 0; i < n; i++) {
+  if (!march && !tma && !group && b->tune.threads > 512) b->tune.threads = 512;
+  for (int i = 0; i < n && !march; i++) {
     rt_handle* h = b->mem[qm[i]];
     StepTuning tn = b->tune;
     for (int par = 0; par < 2; par++) {
@@ -739,7 +755,7 @@ static int batch_build(rt_batch* b) {
                                 : (tma ? tma_path_smem<T>(h->d) : plane_smem<T>(h->d)));
     b->cur0[qm[i]] = h->cur;
   }
-  if (n > 0) {
+  if (n > 0 && !march) {
     const int nall = (int)b->mem.size();
     for (int par = 0; par < 2; par++) {
       if (!b->d_mem[par]) BCUDA_TRY(b, cudaMalloc(&b->d_mem[par], (size_t)nall * sizeof(BatchMember<T>)));

@@ -153,6 +153,13 @@ cudaError_t launch_batch_fused(const BatchFused& F, int grid, int ga, cudaStream
 // rt_persist.cu, rt_persist_w2.cu); done = false when the tuning
 // does not select one of them or the shape does not fit them
 cudaError_t launch_persist(const StepArgs<float>& A, const StepTuning& tn, cudaStream_t st, bool& done);
+// binary32 step of threads marching along k (rt_march.cu): any extents, up
+// to 2^30 cells
+bool march_ok(const Dims& d);
+cudaError_t launch_march(const StepArgs<float>& A, const StepTuning& tn, cudaStream_t st);
+// one step of n fields, in march_batch_launches(n) launches
+int march_batch_launches(int n);
+cudaError_t launch_march_batch(const StepArgs<float>* A, int n, int band, int sweep, cudaStream_t st);
 // bit-exact binary64 step without binary64 divisions (rt_exact.cu).  Flux
 // fields of a two-pass step: f[a] (the cell's right face) and f0[a] (the
 // face-0 plane, the layout of vlo[a])

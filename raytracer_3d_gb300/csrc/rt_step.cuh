@@ -178,7 +178,9 @@ __host__ __device__ __forceinline__ unsigned sr_bits(long long p, unsigned seed)
 // |err| / gap, using the top 24 bits of rnd
 __host__ __device__ __forceinline__ float sr_round(float s, float err, unsigned rnd) {
   const unsigned sb = f32_bits(s);
-  const unsigned nbits = ((err > 0.f) == ((sb >> 31) == 0u)) ? sb + 1u : sb - 1u;
+  // away from zero where err and s have one sign, towards it otherwise (an
+  // err of zero never takes the neighbour)
+  const unsigned nbits = sb + (unsigned)((int)(f32_bits(err) ^ sb) >> 31 | 1);
   const float nb = f32_from_bits(nbits);
   const float gap = fabsf(nb - s);
   const float u = (float)(rnd >> 8) * 5.9604645e-08f;   // [0, 1) in steps of 2^-24
