@@ -63,6 +63,7 @@ struct rt_handle {
   double* vol3 = nullptr;       // 8 x nvol3 wavenumber integrals
   double* result = nullptr;     // DIAG_RESULT_NV doubles
   int* status = nullptr;        // device flag raised by a timed-out wait
+  unsigned* counter = nullptr;  // arrivals at the grid-wide waits of a many-step launch
   unsigned* seed = nullptr;     // binary32 stochastic-rounding seeds, one per ping-pong buffer
   void* pinned = nullptr;       // host staging of one interior field
   int host_direct = 1;          // 1: the GPU reads / writes host arrays itself when the device can
@@ -302,6 +303,14 @@ static bool slab_scratch(rt_handle* h) {
   return true;
 }
 
+// the bit-exact binary64 step of every variant that does not name one of the
+// plane kernels (rt_exact.cu)
+static bool exact_variant(const rt_handle* h) {
+  const int v = h->tune.variant;
+  return h->p.precision == RT_FP64 && !(v == RT_VARIANT_FAST && fast_ready(h)) && v != RT_VARIANT_PLANE &&
+         v != RT_VARIANT_CELL && v != RT_VARIANT_GROUP && h->d.ncell < (1ll << 31);
+}
+
 // one step of the handle from buffer src into 1 - src; returns the kernels launched
 static cudaError_t step_once(rt_handle* h, int src, int* nlaunch) {
   if (h->p.precision == RT_FP64) {
@@ -315,12 +324,10 @@ static cudaError_t step_once(rt_handle* h, int src, int* nlaunch) {
     }
     cudaError_t e = ensure_uc(h, 0);
     if (e != cudaSuccess) return e;
-    // the bit-exact step of every variant that does not name one of the
-    // plane kernels (rt_exact.cu)
-    const int v = h->tune.variant;
-    if (v != RT_VARIANT_PLANE && v != RT_VARIANT_CELL && v != RT_VARIANT_GROUP && h->d.ncell < (1ll << 31)) {
+    if (exact_variant(h)) {
       *nlaunch = 1;
-      if (!exact_in_slabs(h->d)) return launch_step_exact_cells(make_step_args<double>(h, src), h->st);
+      if (!exact_in_slabs(h->d))
+        return launch_step_exact_small(make_step_args<double>(h, src), 1, RT_FORCING_NONE, nullptr, 0.0, nullptr, h->st);
       if (slab_scratch(h)) return launch_step_exact_slabs(make_step_args<double>(h, src), h->slab, h->st, nlaunch);
     }
     *nlaunch = 1;
@@ -1115,7 +1122,8 @@ int rt_create(const rt_dims* dims, const rt_params* params, rt_handle** out) {
   if ((rc = dev_alloc(h, (void**)&h->scratch, h->scratch_len * sizeof(double)))) return bail(rc);
   if ((rc = dev_alloc(h, (void**)&h->vol3, 8 * d.nvol3 * sizeof(double)))) return bail(rc);
   if ((rc = dev_alloc(h, (void**)&h->result, 32 * sizeof(double)))) return bail(rc);
-  if ((rc = dev_alloc(h, (void**)&h->status, sizeof(int)))) return bail(rc);
+  if ((rc = dev_alloc(h, (void**)&h->status, 2 * sizeof(int)))) return bail(rc);
+  h->counter = (unsigned*)h->status + 1;
   if (cudaMemset(h->status, 0, sizeof(int)) != cudaSuccess) return bail(fail(h, RT_ERR_CUDA, "memset"));
   if ((rc = dev_alloc(h, (void**)&h->seed, 2 * sizeof(unsigned)))) return bail(rc);
   if (cudaMemset(h->seed, 0, 2 * sizeof(unsigned)) != cudaSuccess) return bail(fail(h, RT_ERR_CUDA, "memset"));
@@ -1432,7 +1440,25 @@ int rt_integrate(rt_handle* h, int nsteps) {
   if (nsteps < 0) return fail(h, RT_ERR_ARG, "rt_integrate: nsteps < 0");
   if (!h->have_coeff) return fail(h, RT_ERR_STATE, "rt_integrate: rt_calc_parameter first");
   if (!h->have_state) return fail(h, RT_ERR_STATE, "rt_integrate: rt_set_state first");
-  for (int t = 0; t < nsteps; t++) {
+  // small binary64 fields: many steps, and the forcing between them, in one
+  // launch (a wait across the GPU costs 1.2 us, a launch 2)
+  int left = nsteps;
+  while (left >= 4 && exact_variant(h) && !exact_in_slabs(h->d)) {
+    const int n = std::min(left, 1024);
+    cudaError_t e = ensure_uc(h, 0);
+    if (e == cudaSuccess)
+      e = launch_step_exact_small(make_step_args<double>(h, h->cur), n, h->forcing, h->force, h->dzt1, h->counter, h->st);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {   // not all SMs are ours: a launch per step
+      cudaGetLastError();
+      break;
+    }
+    h->launches += 1;
+    if (e != cudaSuccess) return fail(h, RT_ERR_CUDA, "step launch: %s", cudaGetErrorString(e));
+    h->cur ^= n & 1;
+    h->steps_since_set += n;
+    left -= n;
+  }
+  for (int t = 0; t < left; t++) {
     cudaError_t e;
     if (h->forcing != RT_FORCING_NONE) {
       e = apply_forcing(h, h->cur, h->st);

@@ -1,9 +1,9 @@
 // rt_exact.cu -- bit-exact binary64 step without binary64 divisions
 // (arithmetic in rt_exact.cuh), in two forms:
 //
-//   exact_cell_kernel    one launch, one thread per cell, both faces of every
-//                        axis: small fields, where the launch and the latency
-//                        of one pass are the cost;
+//   exact_small_kernel   small fields: one CTA per SM over a range of cells,
+//                        fluxes through shared memory, one step or many in one
+//                        launch (a grid-wide wait between them);
 //   exact_flux_kernel,   two passes that evaluate every face flux once, as the
 //   exact_update_kernel  reference does, over slabs of the slowest axis: the
 //                        flux fields of one slab stay in L2 between the passes
@@ -19,6 +19,9 @@
 // ms, and a CTA of 512 threads per x-y plane 280 us for a 40x120 column
 // (one launch here: 8.2 us), 6.3 ms for a 10x20x60x60 section (97 us) and
 // 8.7 ms for 8x8x16x16^3 (0.74 ms).
+#include <algorithm>
+
+#include "../../include/rt_gb300.h"
 #include "rt_exact.cuh"
 #include "rt_fast.cuh"
 #include "rt_kernels.h"
@@ -81,40 +84,153 @@ __device__ __forceinline__ bool face0_is_copy(const Dims& d, int a) { return a !
 __device__ __forceinline__ double exact_update(const StepArgs<double>& A, int p, double e0, double dE) {
   const Dims& d = A.d;
   double mf = 0.;
-  if (d.n[0] > 1) mf = dmul(e0, __ldcs(A.lam[0] + p));
-  if (d.n[1] > 1) mf = dadd(mf, dmul(e0, __ldcs(A.lam[1] + p)));
-  if (d.n[2] > 1) mf = dadd(mf, dmul(e0, __ldcs(A.lam[2] + p)));
+  if (d.n[0] > 1) mf = dmul(e0, A.lam[0][p]);
+  if (d.n[1] > 1) mf = dadd(mf, dmul(e0, A.lam[1][p]));
+  if (d.n[2] > 1) mf = dadd(mf, dmul(e0, A.lam[2][p]));
   return dadd(e0, dmul(A.dt, dsub(dE, mf)));
 }
 
-__global__ void __launch_bounds__(128) exact_cell_kernel(StepArgs<double> A, CellGeom G) {
-  const Dims& d = A.d;
-  const unsigned pu = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pu >= G.ncell) return;
-  const int p = (int)pu;
-  int c[6];
-  cell_coords(G, pu, c);
-  const double e0 = A.E[p];
-  double dE = 0.;
-#pragma unroll
-  for (int a = 0; a < 6; a++) {
-    if (d.n[a] <= 1) continue;
-    const int ca = c[a];
-    const double Em1 = A.E[nb32(d, G, p, a, ca, -1, c[5])];
-    const double Ep1 = A.E[nb32(d, G, p, a, ca, +1, c[5])];
-    const double Ep2 = A.E[nb32(d, G, p, a, ca, +2, c[5])];
-    const double fr = flux_exact(A.vel[a][p], A.uc[a][p], Em1, e0, Ep1, Ep2);
-    double fl;
-    if (ca > 0 || !face0_is_copy(d, a)) {
-      const int q = ca > 0 ? p - G.s[a] : plane32(G, a, c);
-      const double vl = ca > 0 ? A.vel[a][q] : A.vlo[a][q], ul = ca > 0 ? A.uc[a][q] : A.ucl[a][q];
-      fl = flux_exact(vl, ul, A.E[nb32(d, G, p, a, ca, -2, c[5])], Em1, e0, Ep1);
-    } else {
-      fl = dmul(A.vlo[a][plane32(G, a, c)], e0);
+// ---- small fields: CTA b owns the cells [b*C, (b+1)*C) ----
+// Its face fluxes go through shared memory, evaluated once: list a holds the
+// left-face fluxes of the first sh = min(stride, C) cells (right-face fluxes
+// of cells before the CTA's) and then the right-face fluxes of all C, so
+// cell i has its left flux at i and its right flux at i + sh.  One more list
+// holds the reflected z face 0 of the cells that have it.
+struct SmallGeom {
+  CellGeom G;
+  int C;
+  int axes, axis[6];             // axes with n > 1
+  int sh[6], start[8];           // by position in axis[]; start[axes]: the z face-0 list, start[axes + 1]: the end
+  DivU32 sdiv[6], ndiv[6];       // stride and extent of every axis
+};
+
+struct Forcing {
+  int kind;                      // RT_FORCING_NONE: none between the steps
+  const double* F;
+  double dz;
+  DivU32 s3;                     // cells of a (k,l,m) volume
+};
+
+__device__ __forceinline__ int coord(const SmallGeom& S, int a, unsigned p) {
+  const unsigned q = S.sdiv[a].div(p);
+  return (int)(q - S.ndiv[a].div(q) * S.ndiv[a].d);
+}
+
+// set_forcing on one cell of the bottom plane, as forcing_kernel does
+__device__ __forceinline__ double forced(const StepArgs<double>& A, const Forcing& W, int p, double e) {
+  const unsigned sp = W.s3.div((unsigned)p);
+  const int nxy = A.d.n[0] * A.d.n[1];
+  const double f = W.F[(p - (int)(sp * W.s3.d)) + (int)sp * nxy];
+  if (W.kind == RT_FORCING_FLUX) return dadd(e, div_rn(dmul(A.dt, f), W.dz));
+  const double w = fmax2(0.0, A.vel[2][p]);
+  return dsub(e, div_rn(dmul(dmul(A.dt, w), dsub(e, f)), W.dz));
+}
+
+// all CTAs of the launch (a cooperative one) have passed their `round`-th
+// call; false when the wait ran out (status raised, every CTA leaves)
+__device__ __forceinline__ bool grid_wait(unsigned* counter, unsigned round, int* status, int* ok) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(counter, 1u);
+    const unsigned target = round * gridDim.x;
+    bool there = false;
+    for (unsigned it = 0; it < (1u << 22) && !there; it++) {
+      unsigned v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
+      there = v >= target;
     }
-    dE = dsub(dE, div_rn(dsub(fr, fl), A.g.d[a][pidx(ca + 1)]));
+    if (!there) atomicOr(status, 1);
+    *ok = there ? 1 : 0;
   }
-  A.Enew[p] = exact_update(A, p, e0, dE);
+  __syncthreads();
+  return *ok != 0;
+}
+
+// nsteps steps from A.E (and back and forth between the two buffers); with
+// more than one the launch is cooperative and `counter` starts at zero.  The
+// forcing acts before every step: on A.E at the start, then on each new
+// state but the last as it is stored.
+__global__ void __launch_bounds__(512) exact_small_kernel(const __grid_constant__ StepArgs<double> A,
+                                                          const __grid_constant__ SmallGeom S,
+                                                          const __grid_constant__ Forcing W, int nsteps,
+                                                          unsigned* counter) {
+  extern __shared__ double sF[];
+  __shared__ int ok;
+  const Dims& d = A.d;
+  const CellGeom& G = S.G;
+  const int p0 = (int)blockIdx.x * S.C;
+  const int count = (int)G.ncell - p0 < S.C ? (int)G.ncell - p0 : S.C;
+  double* E = const_cast<double*>(A.E);
+  double* En = A.Enew;
+  unsigned round = 0;
+  if (nsteps > 1 && W.kind != RT_FORCING_NONE) {
+    for (int i = threadIdx.x; i < count; i += blockDim.x)
+      if (coord(S, 2, (unsigned)(p0 + i)) == 0) E[p0 + i] = forced(A, W, p0 + i, E[p0 + i]);
+    if (!grid_wait(counter, ++round, A.status, &ok)) return;
+  }
+  for (int t = 0; t < nsteps; t++) {
+    // ---- fluxes ----
+    for (int j = threadIdx.x; j < S.start[S.axes + 1]; j += blockDim.x) {
+      int f = 0;
+      while (j >= S.start[f + 1]) f++;
+      const int i = j - S.start[f];
+      if (f < S.axes) {
+        const int a = S.axis[f], s = G.s[a], sh = S.sh[f];
+        const int owner = i < sh ? i : i - sh;           // the CTA's cell this flux is for
+        if (owner >= count) continue;
+        const int q = i < sh ? p0 + i - s : p0 + i - sh; // its right face
+        if (q < 0) continue;
+        const int ca = coord(S, a, (unsigned)q);
+        if (i < sh && ca == d.n[a] - 1) continue;        // the owner has face 0 on its left
+        const int cm = a == 2 ? coord(S, 5, (unsigned)q) : 0;
+        const double Em1 = __ldcg(E + nb32(d, G, q, a, ca, -1, cm));
+        const double Ep1 = __ldcg(E + nb32(d, G, q, a, ca, +1, cm));
+        const double Ep2 = __ldcg(E + nb32(d, G, q, a, ca, +2, cm));
+        sF[j] = flux_exact(A.vel[a][q], A.uc[a][q], Em1, __ldcg(E + q), Ep1, Ep2);
+      } else {
+        const int p = p0 + i;
+        if (i >= count || coord(S, 2, (unsigned)p) != 0) continue;
+        int c[6];
+        cell_coords(G, (unsigned)p, c);
+        const int q = plane32(G, 2, c);
+        sF[j] = flux_exact(A.vlo[2][q], A.ucl[2][q], __ldcg(E + nb32(d, G, p, 2, 0, -2, c[5])),
+                           __ldcg(E + nb32(d, G, p, 2, 0, -1, c[5])), __ldcg(E + p),
+                           __ldcg(E + nb32(d, G, p, 2, 0, +1, c[5])));
+      }
+    }
+    __syncthreads();
+    // ---- divergence and update ----
+    for (int i = threadIdx.x; i < count; i += blockDim.x) {
+      const int p = p0 + i;
+      int c[6];
+      cell_coords(G, (unsigned)p, c);
+      const double e0 = __ldcg(E + p);
+      double dE = 0.;
+#pragma unroll
+      for (int f = 0; f < 6; f++) {
+        if (f >= S.axes) break;
+        const int a = S.axis[f];
+        int ca = 0;
+#pragma unroll
+        for (int b = 0; b < 6; b++) ca = b == a ? c[b] : ca;
+        const double fr = sF[S.start[f] + S.sh[f] + i];
+        double fl;
+        if (ca > 0) fl = sF[S.start[f] + i];
+        else if (face0_is_copy(d, a)) fl = dmul(A.vlo[a][plane32(G, a, c)], e0);
+        else fl = sF[S.start[S.axes] + i];
+        dE = dsub(dE, div_rn(dsub(fr, fl), A.g.d[a][pidx(ca + 1)]));
+      }
+      double e = exact_update(A, p, e0, dE);
+      if (W.kind != RT_FORCING_NONE && t + 1 < nsteps && c[2] == 0) e = forced(A, W, p, e);
+      En[p] = e;
+    }
+    if (t + 1 == nsteps) return;
+    if (!grid_wait(counter, ++round, A.status, &ok)) return;
+    double* x = E;
+    E = En;
+    En = x;
+  }
 }
 
 // ---- the two passes over a slab: values [c0, c0 + count) of the slowest
@@ -225,9 +341,60 @@ long long exact_scratch_z0(const Dims& d) {
   return ax == 2 ? d.s[2] : exact_slab_planes(d) * (d.s[ax] / d.n[2]);
 }
 
-cudaError_t launch_step_exact_cells(const StepArgs<double>& A, cudaStream_t st) {
-  exact_cell_kernel<<<(unsigned)((A.d.ncell + 127) / 128), 128, 0, st>>>(A, make_cells(A.d));
-  return cudaGetLastError();
+namespace {
+
+// cells per CTA: one CTA per SM, so that the binary64 work spreads evenly
+SmallGeom make_small(const Dims& d, int ctas) {
+  SmallGeom S;
+  S.G = make_cells(d);
+  S.C = (int)((d.ncell + ctas - 1) / ctas);
+  S.axes = 0;
+  int at = 0;
+  for (int a = 0; a < 6; a++) {
+    S.sdiv[a] = make_div((unsigned)d.s[a]);
+    S.ndiv[a] = make_div((unsigned)d.n[a]);
+    if (d.n[a] <= 1) continue;
+    const int f = S.axes++;
+    S.axis[f] = a;
+    S.sh[f] = d.s[a] < S.C ? (int)d.s[a] : S.C;
+    S.start[f] = at;
+    at += S.sh[f] + S.C;
+  }
+  S.start[S.axes] = at;
+  if (d.n[2] > 1 && d.lower_refl) at += S.C;
+  S.start[S.axes + 1] = at;
+  return S;
+}
+
+int sm_count() {
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return n;
+}
+
+}  // namespace
+
+cudaError_t launch_step_exact_small(const StepArgs<double>& A, int nsteps, int forcing, const double* F, double dz,
+                                    unsigned* counter, cudaStream_t st) {
+  const SmallGeom S = make_small(A.d, sm_count());
+  const int jobs = S.start[S.axes + 1];
+  const int threads = jobs <= 128 ? 128 : (jobs <= 256 ? 256 : 512);
+  const size_t sm = (size_t)jobs * sizeof(double);
+  Forcing W{forcing, F, dz, make_div((unsigned)A.d.s[3])};
+  const unsigned ctas = (unsigned)((A.d.ncell + S.C - 1) / S.C);
+  cudaError_t e = cudaFuncSetAttribute(exact_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
+  if (nsteps == 1) {
+    exact_small_kernel<<<ctas, threads, sm, st>>>(A, S, W, 1, nullptr);
+    return cudaGetLastError();
+  }
+  e = cudaMemsetAsync(counter, 0, sizeof(unsigned), st);
+  if (e != cudaSuccess) return e;
+  StepArgs<double> a = A;
+  SmallGeom s = S;
+  void* args[] = {&a, &s, &W, &nsteps, &counter};
+  return cudaLaunchCooperativeKernel((const void*)exact_small_kernel, dim3(ctas), dim3((unsigned)threads), args, sm, st);
 }
 
 cudaError_t launch_step_exact_slabs(const StepArgs<double>& A, const SplitFluxes& F, cudaStream_t st, int* nlaunch) {

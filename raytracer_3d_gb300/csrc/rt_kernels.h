@@ -168,11 +168,15 @@ struct SplitFluxes {
   double* f0[6];
 };
 // fields of more cells take the two passes over slabs, the others one launch
+// per step, or for nsteps of them with the forcing in between (RT_FORCING_*
+// of rt_gb300.h, counter: one unsigned of device memory; a single step leaves
+// the forcing to the caller)
 bool exact_in_slabs(const Dims& d);
 // doubles of the slab scratch: flux field of axis a, and the face-0 plane of z
 long long exact_scratch(const Dims& d, int a);
 long long exact_scratch_z0(const Dims& d);
-cudaError_t launch_step_exact_cells(const StepArgs<double>& A, cudaStream_t st);
+cudaError_t launch_step_exact_small(const StepArgs<double>& A, int nsteps, int forcing, const double* F, double dz,
+                                    unsigned* counter, cudaStream_t st);
 cudaError_t launch_step_exact_slabs(const StepArgs<double>& A, const SplitFluxes& F, cudaStream_t st, int* nlaunch);
 // fast binary64 step (rt_fast.cu): the flux fields of the two-pass step,
 // h = |v|/2*(1-|v dt/d|) per face (hr: right faces, hl: face-0 planes),

@@ -61,3 +61,41 @@ def test_forms_equal_the_cell_kernel(n, walls):
         m.close()
     assert np.isfinite(got[0]).all()
     assert np.array_equal(got[1], got[0]) and np.array_equal(got[2], got[0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("walls", [True, False])
+@pytest.mark.parametrize("forcing", ["none", "flux", "relax"])
+@pytest.mark.parametrize("n", [(1, 1, 40, 1, 1, 120), (6, 5, 6, 4, 4, 6), (2, 2, 2, 2, 2, 2), (1, 9, 6, 1, 12, 100),
+                               (7, 3, 5, 2, 6, 4), (1, 1, 2, 1, 1, 4), (300, 1, 1, 8, 1, 2)])
+def test_many_steps_in_one_launch(n, forcing, walls):
+    """nine steps in one launch, and as launches of one step, against the
+    one-thread-per-cell kernel with its forcing kernel before every step"""
+    import __graft_entry__ as g
+    g.build()
+    rng = np.random.default_rng(6)
+    exp = configs.shear_mini(n=n, upper=walls, lower=walls)
+    exp.fixed = (1e-3, 0.0, 1e-2)
+    E0 = rng.random(n) ** 4 * 1e-3
+    sl = (slice(2, -2),) * 6
+    got = []
+    for variant, parts in (("cell", (9,)), ("tma", (9,)), ("tma", (1,) * 9), ("tma", (4, 5))):
+        m = configs.build_model(exp, "fp64")
+        m.E[sl] = E0
+        m.set_state()
+        if forcing != "none":
+            m.set_forcing(forcing, np.asfortranarray(np.random.default_rng(7).random(m.forcing_shape()) * 1e-4))
+        m.set_tuning(variant, 8, 256)
+        l0 = m.launch_count()
+        for k in parts:
+            m.integrate(k)
+        launches = m.launch_count() - l0
+        E = m.get_state()[sl].copy()
+        b, f = m.diagnose()
+        got.append((E, [b["eint"], b["mflint"], b["mfl_max"]] + [f[q].copy() for q in sorted(f)]))
+        m.close()
+        if variant == "tma":
+            assert launches == (len(parts) if len(parts) < 9 else (9 if forcing == "none" else 18))
+    for E, b in got[1:]:
+        assert np.array_equal(E, got[0][0])
+        assert all(np.array_equal(x, y) for x, y in zip(b, got[0][1]))
