@@ -147,83 +147,165 @@ __device__ __forceinline__ bool grid_wait(unsigned* counter, unsigned round, int
   return *ok != 0;
 }
 
+// what a thread knows of one face flux for the whole launch
+struct FaceJob {
+  bool live;
+  int at, q, m1, p1, p2;   // slot; cell left of the face and its neighbours
+  double v, u;
+};
+__device__ __forceinline__ FaceJob face_job(const StepArgs<double>& A, const SmallGeom& S, int p0, int count, int j) {
+  const Dims& d = A.d;
+  const CellGeom& G = S.G;
+  FaceJob J;
+  J.live = false;
+  if (j >= S.start[S.axes + 1]) return J;
+  int f = 0;
+  while (j >= S.start[f + 1]) f++;
+  const int i = j - S.start[f];
+  J.at = j;
+  if (f < S.axes) {
+    const int a = S.axis[f], s = G.s[a], sh = S.sh[f];
+    const int owner = i < sh ? i : i - sh;               // the CTA's cell this flux is for
+    const int q = i < sh ? p0 + i - s : p0 + i - sh;     // its right face
+    if (owner >= count || q < 0) return J;
+    const int ca = coord(S, a, (unsigned)q);
+    if (i < sh && ca == d.n[a] - 1) return J;            // the owner has face 0 on its left
+    const int cm = a == 2 ? coord(S, 5, (unsigned)q) : 0;
+    J.q = q;
+    J.m1 = nb32(d, G, q, a, ca, -1, cm);
+    J.p1 = nb32(d, G, q, a, ca, +1, cm);
+    J.p2 = nb32(d, G, q, a, ca, +2, cm);
+    J.v = A.vel[a][q];
+    J.u = A.uc[a][q];
+  } else {                                               // reflected z face 0
+    const int p = p0 + i;
+    if (i >= count || coord(S, 2, (unsigned)p) != 0) return J;
+    int c[6];
+    cell_coords(G, (unsigned)p, c);
+    const int r = plane32(G, 2, c);
+    J.q = nb32(d, G, p, 2, 0, -1, c[5]);
+    J.m1 = nb32(d, G, p, 2, 0, -2, c[5]);
+    J.p1 = p;
+    J.p2 = nb32(d, G, p, 2, 0, +1, c[5]);
+    J.v = A.vlo[2][r];
+    J.u = A.ucl[2][r];
+  }
+  J.live = true;
+  return J;
+}
+__device__ __forceinline__ void face_run(const FaceJob& J, const double* E, double* sF) {
+  if (!J.live) return;
+  sF[J.at] = flux_exact(J.v, J.u, __ldcg(E + J.m1), __ldcg(E + J.q), __ldcg(E + J.p1), __ldcg(E + J.p2));
+}
+
+// and of one cell: its axes' spacing, and the slots of its two fluxes (left
+// -1: v*E with the face-0 velocity)
+template <int AX>
+struct CellJob {
+  bool live, bottom;
+  int p;
+  int right[AX], left[AX];
+  double dd[AX], v0[AX], lam[3];
+};
+template <int AX>
+__device__ __forceinline__ CellJob<AX> cell_job(const StepArgs<double>& A, const SmallGeom& S, int p0, int count, int i) {
+  const Dims& d = A.d;
+  CellJob<AX> J;
+  J.live = i < count;
+  if (!J.live) return J;
+  J.p = p0 + i;
+  int c[6];
+  cell_coords(S.G, (unsigned)J.p, c);
+  J.bottom = c[2] == 0;
+#pragma unroll
+  for (int f = 0; f < AX; f++) {
+    if (f >= S.axes) break;
+    const int a = S.axis[f];
+    int ca = 0;
+#pragma unroll
+    for (int b = 0; b < 6; b++) ca = b == a ? c[b] : ca;
+    J.right[f] = S.start[f] + S.sh[f] + i;
+    J.left[f] = ca > 0 ? S.start[f] + i : (face0_is_copy(d, a) ? -1 : S.start[S.axes] + i);
+    J.v0[f] = J.left[f] < 0 ? A.vlo[a][plane32(S.G, a, c)] : 0.0;
+    J.dd[f] = A.g.d[a][pidx(ca + 1)];
+  }
+#pragma unroll
+  for (int k = 0; k < 3; k++) J.lam[k] = d.n[k] > 1 ? A.lam[k][J.p] : 0.0;
+  return J;
+}
+template <int AX>
+__device__ __forceinline__ void cell_run(const StepArgs<double>& A, const SmallGeom& S, const Forcing& W,
+                                         const CellJob<AX>& J, const double* E, double* En, const double* sF,
+                                         bool force) {
+  if (!J.live) return;
+  const Dims& d = A.d;
+  const double e0 = __ldcg(E + J.p);
+  double q[AX];   // the axes' quotients do not depend on one another
+#pragma unroll
+  for (int f = 0; f < AX; f++) {
+    if (f >= S.axes) break;
+    const double fl = J.left[f] >= 0 ? sF[J.left[f]] : dmul(J.v0[f], e0);
+    q[f] = div_rn(dsub(sF[J.right[f]], fl), J.dd[f]);
+  }
+  double dE = 0.;
+#pragma unroll
+  for (int f = 0; f < AX; f++) {
+    if (f >= S.axes) break;
+    dE = dsub(dE, q[f]);
+  }
+  double mf = 0.;
+  if (d.n[0] > 1) mf = dmul(e0, J.lam[0]);
+  if (d.n[1] > 1) mf = dadd(mf, dmul(e0, J.lam[1]));
+  if (d.n[2] > 1) mf = dadd(mf, dmul(e0, J.lam[2]));
+  double e = dadd(e0, dmul(A.dt, dsub(dE, mf)));
+  if (force && J.bottom) e = forced(A, W, J.p, e);
+  En[J.p] = e;
+}
+
 // nsteps steps from A.E (and back and forth between the two buffers); with
 // more than one the launch is cooperative and `counter` starts at zero.  The
 // forcing acts before every step: on A.E at the start, then on each new
 // state but the last as it is stored.
+// K > 0: a thread has at most K faces and one cell (and the field at most AX
+// axes), whose indices and coefficients it keeps in registers from step to
+// step; K = 0: it works them out anew.
+template <int K, int AX>
 __global__ void __launch_bounds__(512) exact_small_kernel(const __grid_constant__ StepArgs<double> A,
                                                           const __grid_constant__ SmallGeom S,
                                                           const __grid_constant__ Forcing W, int nsteps,
                                                           unsigned* counter) {
   extern __shared__ double sF[];
   __shared__ int ok;
-  const Dims& d = A.d;
-  const CellGeom& G = S.G;
   const int p0 = (int)blockIdx.x * S.C;
-  const int count = (int)G.ncell - p0 < S.C ? (int)G.ncell - p0 : S.C;
+  const int count = (int)S.G.ncell - p0 < S.C ? (int)S.G.ncell - p0 : S.C;
   double* E = const_cast<double*>(A.E);
   double* En = A.Enew;
   unsigned round = 0;
-  if (nsteps > 1 && W.kind != RT_FORCING_NONE) {
+  const bool forcing = W.kind != RT_FORCING_NONE;
+  FaceJob face[K > 0 ? K : 1];
+  CellJob<AX> cell;
+  if constexpr (K > 0) {
+#pragma unroll
+    for (int k = 0; k < K; k++) face[k] = face_job(A, S, p0, count, (int)(threadIdx.x + k * blockDim.x));
+    cell = cell_job<AX>(A, S, p0, count, (int)threadIdx.x);
+  }
+  if (nsteps > 1 && forcing) {
     for (int i = threadIdx.x; i < count; i += blockDim.x)
       if (coord(S, 2, (unsigned)(p0 + i)) == 0) E[p0 + i] = forced(A, W, p0 + i, E[p0 + i]);
     if (!grid_wait(counter, ++round, A.status, &ok)) return;
   }
   for (int t = 0; t < nsteps; t++) {
-    // ---- fluxes ----
-    for (int j = threadIdx.x; j < S.start[S.axes + 1]; j += blockDim.x) {
-      int f = 0;
-      while (j >= S.start[f + 1]) f++;
-      const int i = j - S.start[f];
-      if (f < S.axes) {
-        const int a = S.axis[f], s = G.s[a], sh = S.sh[f];
-        const int owner = i < sh ? i : i - sh;           // the CTA's cell this flux is for
-        if (owner >= count) continue;
-        const int q = i < sh ? p0 + i - s : p0 + i - sh; // its right face
-        if (q < 0) continue;
-        const int ca = coord(S, a, (unsigned)q);
-        if (i < sh && ca == d.n[a] - 1) continue;        // the owner has face 0 on its left
-        const int cm = a == 2 ? coord(S, 5, (unsigned)q) : 0;
-        const double Em1 = __ldcg(E + nb32(d, G, q, a, ca, -1, cm));
-        const double Ep1 = __ldcg(E + nb32(d, G, q, a, ca, +1, cm));
-        const double Ep2 = __ldcg(E + nb32(d, G, q, a, ca, +2, cm));
-        sF[j] = flux_exact(A.vel[a][q], A.uc[a][q], Em1, __ldcg(E + q), Ep1, Ep2);
-      } else {
-        const int p = p0 + i;
-        if (i >= count || coord(S, 2, (unsigned)p) != 0) continue;
-        int c[6];
-        cell_coords(G, (unsigned)p, c);
-        const int q = plane32(G, 2, c);
-        sF[j] = flux_exact(A.vlo[2][q], A.ucl[2][q], __ldcg(E + nb32(d, G, p, 2, 0, -2, c[5])),
-                           __ldcg(E + nb32(d, G, p, 2, 0, -1, c[5])), __ldcg(E + p),
-                           __ldcg(E + nb32(d, G, p, 2, 0, +1, c[5])));
-      }
-    }
-    __syncthreads();
-    // ---- divergence and update ----
-    for (int i = threadIdx.x; i < count; i += blockDim.x) {
-      const int p = p0 + i;
-      int c[6];
-      cell_coords(G, (unsigned)p, c);
-      const double e0 = __ldcg(E + p);
-      double dE = 0.;
+    const bool force = forcing && t + 1 < nsteps;
+    if constexpr (K > 0) {
 #pragma unroll
-      for (int f = 0; f < 6; f++) {
-        if (f >= S.axes) break;
-        const int a = S.axis[f];
-        int ca = 0;
-#pragma unroll
-        for (int b = 0; b < 6; b++) ca = b == a ? c[b] : ca;
-        const double fr = sF[S.start[f] + S.sh[f] + i];
-        double fl;
-        if (ca > 0) fl = sF[S.start[f] + i];
-        else if (face0_is_copy(d, a)) fl = dmul(A.vlo[a][plane32(G, a, c)], e0);
-        else fl = sF[S.start[S.axes] + i];
-        dE = dsub(dE, div_rn(dsub(fr, fl), A.g.d[a][pidx(ca + 1)]));
-      }
-      double e = exact_update(A, p, e0, dE);
-      if (W.kind != RT_FORCING_NONE && t + 1 < nsteps && c[2] == 0) e = forced(A, W, p, e);
-      En[p] = e;
+      for (int k = 0; k < K; k++) face_run(face[k], E, sF);
+      __syncthreads();
+      cell_run<AX>(A, S, W, cell, E, En, sF, force);
+    } else {
+      for (int j = threadIdx.x; j < S.start[S.axes + 1]; j += blockDim.x) face_run(face_job(A, S, p0, count, j), E, sF);
+      __syncthreads();
+      for (int i = threadIdx.x; i < count; i += blockDim.x)
+        cell_run<AX>(A, S, W, cell_job<AX>(A, S, p0, count, i), E, En, sF, force);
     }
     if (t + 1 == nsteps) return;
     if (!grid_wait(counter, ++round, A.status, &ok)) return;
@@ -383,10 +465,17 @@ cudaError_t launch_step_exact_small(const StepArgs<double>& A, int nsteps, int f
   const size_t sm = (size_t)jobs * sizeof(double);
   Forcing W{forcing, F, dz, make_div((unsigned)A.d.s[3])};
   const unsigned ctas = (unsigned)((A.d.ncell + S.C - 1) / S.C);
-  cudaError_t e = cudaFuncSetAttribute(exact_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  // many steps keep what they know where it fits: fields of two active axes
+  // (columns, whose steps are all latency)
+  void (*kernel)(StepArgs<double>, SmallGeom, Forcing, int, unsigned*) = exact_small_kernel<0, 6>;
+  if (nsteps > 1 && S.axes <= 2 && S.C <= threads) {
+    if (jobs <= threads) kernel = exact_small_kernel<1, 2>;
+    else if (jobs <= 2 * threads) kernel = exact_small_kernel<2, 2>;
+  }
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
   if (nsteps == 1) {
-    exact_small_kernel<<<ctas, threads, sm, st>>>(A, S, W, 1, nullptr);
+    kernel<<<ctas, threads, sm, st>>>(A, S, W, 1, nullptr);
     return cudaGetLastError();
   }
   e = cudaMemsetAsync(counter, 0, sizeof(unsigned), st);
@@ -394,7 +483,7 @@ cudaError_t launch_step_exact_small(const StepArgs<double>& A, int nsteps, int f
   StepArgs<double> a = A;
   SmallGeom s = S;
   void* args[] = {&a, &s, &W, &nsteps, &counter};
-  return cudaLaunchCooperativeKernel((const void*)exact_small_kernel, dim3(ctas), dim3((unsigned)threads), args, sm, st);
+  return cudaLaunchCooperativeKernel((const void*)kernel, dim3(ctas), dim3((unsigned)threads), args, sm, st);
 }
 
 cudaError_t launch_step_exact_slabs(const StepArgs<double>& A, const SplitFluxes& F, cudaStream_t st, int* nlaunch) {
