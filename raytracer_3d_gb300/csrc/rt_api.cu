@@ -60,9 +60,11 @@ struct rt_handle {
   int uc_holds = 0;             // uc/ucl hold 0: uCFL of the bit-exact kernels, 1: h of the fast step
   double* scratch = nullptr;    // reductions
   long long scratch_len = 0;
+  double* coeff_mem = nullptr;  // small fields: scratch of rt_calc_parameter
   double* vol3 = nullptr;       // 8 x nvol3 wavenumber integrals
   double* result = nullptr;     // DIAG_RESULT_NV doubles
   int* status = nullptr;        // device flag raised by a timed-out wait
+  int host_status = 0;          // its value as the last download to the host brought it
   unsigned* counter = nullptr;  // arrivals at the grid-wide waits of a many-step launch
   unsigned* seed = nullptr;     // binary32 stochastic-rounding seeds, one per ping-pong buffer
   void* pinned = nullptr;       // host staging of one interior field
@@ -389,11 +391,14 @@ static int upload_tab32(rt_handle* h) {
 }
 
 // after a synchronisation: report a device-side wait that timed out
+static int status_error(rt_handle* h, int st) {
+  if (st) return fail(h, RT_ERR_CUDA, "a device-side wait timed out (status %d); results are invalid", st);
+  return RT_OK;
+}
 static int check_status(rt_handle* h) {
   int st = 0;
   CUDA_TRY(h, cudaMemcpy(&st, h->status, sizeof(int), cudaMemcpyDeviceToHost));
-  if (st) return fail(h, RT_ERR_CUDA, "a device-side wait timed out (status %d); results are invalid", st);
-  return RT_OK;
+  return status_error(h, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -1142,6 +1147,7 @@ int rt_destroy(rt_handle* h) {
   for (int c = 0; c < 3; c++) cudaFree(h->lam[c]);
   for (int a = 0; a < 6; a++) { cudaFree(h->uc[a]); cudaFree(h->ucl[a]); }
   cudaFree(h->scratch);
+  cudaFree(h->coeff_mem);
   cudaFree(h->vol3);
   cudaFree(h->result);
   cudaFree(h->status);
@@ -1226,13 +1232,21 @@ int rt_calc_parameter(rt_handle* h) {
   const Grid g = make_grid(h);
 
   // scratch of the dispersion relation: a ring of m planes, 256 MB or the
-  // three planes it cannot do without
+  // three planes it cannot do without.  A small one stays with the handle
+  // (taking 1.4 MB from the stream-ordered pool and giving it back cost 0.3 ms)
   double* scratch = nullptr;
   int ring = coeff_ring(d, 256ll << 20);
-  int rc = tmp_alloc(h, (void**)&scratch, (size_t)coeff_scratch(d, ring) * sizeof(double));
-  if (rc && ring > 3) {
-    ring = 3;
+  const bool small = coeff_scratch(d, ring) * (long long)sizeof(double) <= (4ll << 20);
+  int rc = RT_OK;
+  if (small) {
+    if (!h->coeff_mem) rc = dev_alloc(h, (void**)&h->coeff_mem, (size_t)coeff_scratch(d, ring) * sizeof(double));
+    scratch = h->coeff_mem;
+  } else {
     rc = tmp_alloc(h, (void**)&scratch, (size_t)coeff_scratch(d, ring) * sizeof(double));
+    if (rc && ring > 3) {
+      ring = 3;
+      rc = tmp_alloc(h, (void**)&scratch, (size_t)coeff_scratch(d, ring) * sizeof(double));
+    }
   }
   if (rc) return rc;
   int nl = 0;
@@ -1241,7 +1255,7 @@ int rt_calc_parameter(rt_handle* h) {
                       : launch_coeff(d, bg, g, ph, coeff_out<float>(h), scratch, ring, h->result, &nl, h->st);
   h->launches += nl;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&h->rate, h->result, sizeof(double), cudaMemcpyDeviceToHost, h->st);
-  cudaFreeAsync(scratch, h->st);   // stream-ordered: after the kernels
+  if (!small) cudaFreeAsync(scratch, h->st);   // stream-ordered: after the kernels
   const cudaError_t e2 = cudaStreamSynchronize(h->st);
   if (e == cudaSuccess) e = e2;
   if (e != cudaSuccess) return fail(h, RT_ERR_CUDA, "coefficients: %s", cudaGetErrorString(e));
@@ -1323,15 +1337,33 @@ static bool use_host_direct(rt_handle* h) {
   return h->pageable == 1;
 }
 
+// the state from / to the host's padded array by the GPU itself, queued on
+// the handle's stream
+static int queue_gather(rt_handle* h, const double* E) {
+  h->cur = 0;
+  const cudaError_t e = h->p.precision == RT_FP64 ? launch_host_gather<double>(E, (double*)h->E[0], h->d, h->st)
+                                                  : launch_host_gather<float>(E, (float*)h->E[0], h->d, h->st);
+  if (e != cudaSuccess) return fail(h, RT_ERR_CUDA, "host gather: %s", cudaGetErrorString(e));
+  h->launches += 1;
+  return RT_OK;
+}
+static int scatter_and_wait(rt_handle* h, double* E) {
+  const cudaError_t e =
+      h->p.precision == RT_FP64
+          ? launch_host_scatter<double>((const double*)h->E[h->cur], E, h->d, h->status, &h->host_status, h->st)
+          : launch_host_scatter<float>((const float*)h->E[h->cur], E, h->d, h->status, &h->host_status, h->st);
+  if (e != cudaSuccess) return fail(h, RT_ERR_CUDA, "host scatter: %s", cudaGetErrorString(e));
+  h->launches += 1;
+  CUDA_TRY(h, cudaStreamSynchronize(h->st));
+  return status_error(h, h->host_status);
+}
+
 int rt_set_state(rt_handle* h, const double* E) {
   if (!h || !E) return RT_ERR_ARG;
   const Dims& d = h->d;
   if (use_host_direct(h)) {
-    h->cur = 0;
-    cudaError_t e = h->p.precision == RT_FP64 ? launch_host_gather<double>(E, (double*)h->E[0], d, h->st)
-                                              : launch_host_gather<float>(E, (float*)h->E[0], d, h->st);
-    if (e != cudaSuccess) return fail(h, RT_ERR_CUDA, "host gather: %s", cudaGetErrorString(e));
-    h->launches += 1;
+    const int rc = queue_gather(h, E);
+    if (rc) return rc;
     CUDA_TRY(h, cudaStreamSynchronize(h->st));
     h->have_state = true;
     h->steps_since_set = 0;
@@ -1353,15 +1385,7 @@ int rt_get_state(rt_handle* h, double* E) {
   if (!h || !E) return RT_ERR_ARG;
   if (!h->have_state) return fail(h, RT_ERR_STATE, "rt_get_state: no state (rt_set_state first)");
   const Dims& d = h->d;
-  if (use_host_direct(h)) {
-    cudaError_t e = h->p.precision == RT_FP64
-                        ? launch_host_scatter<double>((const double*)h->E[h->cur], E, d, h->st)
-                        : launch_host_scatter<float>((const float*)h->E[h->cur], E, d, h->st);
-    if (e != cudaSuccess) return fail(h, RT_ERR_CUDA, "host scatter: %s", cudaGetErrorString(e));
-    h->launches += 1;
-    CUDA_TRY(h, cudaStreamSynchronize(h->st));
-    return check_status(h);
-  }
+  if (use_host_direct(h)) return scatter_and_wait(h, E);
   int rc = ensure_pinned(h);
   if (rc) return rc;
   CUDA_TRY(h, cudaMemcpyAsync(h->pinned, h->E[h->cur], (size_t)d.ncell * h->elem, cudaMemcpyDeviceToHost, h->st));
@@ -1492,6 +1516,17 @@ int rt_step_dry(rt_handle* h, int nsteps) {
 }
 
 int rt_integrate_host(rt_handle* h, double* E) {
+  if (h && E && h->have_coeff && use_host_direct(h)) {   // upload, step and download queued, one wait
+    int rc = queue_gather(h, E);
+    if (rc) return rc;
+    h->have_state = true;
+    h->steps_since_set = 0;
+    if ((rc = rt_integrate(h, 1))) {
+      cudaStreamSynchronize(h->st);   // the upload may still read the caller's array
+      return rc;
+    }
+    return scatter_and_wait(h, E);
+  }
   int rc = rt_set_state(h, E);
   if (rc) return rc;
   if ((rc = rt_integrate(h, 1))) return rc;

@@ -379,7 +379,10 @@ static dim3 cell_grid(const Dims& d, int threads) {
 // order; the host array is padded by RT_ONX on every axis (Fortran order).
 template <bool TO_DEVICE, class T>
 __global__ void host_rows_kernel(const double* __restrict__ hsrc, double* __restrict__ hdst,
-                                 const T* __restrict__ dsrc, T* __restrict__ ddst, Dims d) {
+                                 const T* __restrict__ dsrc, T* __restrict__ ddst, Dims d,
+                                 const int* __restrict__ status, int* __restrict__ hstatus) {
+  // on the way to the host the wait-timeout flag goes along
+  if (!TO_DEVICE && blockIdx.x == 0 && threadIdx.x == 0) *hstatus = *status;
   long long P[6];
 #pragma unroll
   for (int a = 0; a < 6; a++) P[a] = d.n[a] + 2 * RT_ONX;
@@ -404,20 +407,27 @@ __global__ void host_rows_kernel(const double* __restrict__ hsrc, double* __rest
   }
 }
 
+// a warp per row, 64 resident warps per SM at most
+static unsigned rows_grid(const Dims& d) {
+  const long long blocks = (d.ncell / d.n[0] + 7) / 8;
+  return (unsigned)(blocks < 8 * 152 ? blocks : 8 * 152);
+}
+
 template <class T>
 cudaError_t launch_host_gather(const double* host, T* dst, const Dims& d, cudaStream_t st) {
-  host_rows_kernel<true, T><<<8 * 152, 256, 0, st>>>(host, nullptr, nullptr, dst, d);
+  host_rows_kernel<true, T><<<rows_grid(d), 256, 0, st>>>(host, nullptr, nullptr, dst, d, nullptr, nullptr);
   return cudaGetLastError();
 }
 template <class T>
-cudaError_t launch_host_scatter(const T* src, double* host, const Dims& d, cudaStream_t st) {
-  host_rows_kernel<false, T><<<8 * 152, 256, 0, st>>>(nullptr, host, src, nullptr, d);
+cudaError_t launch_host_scatter(const T* src, double* host, const Dims& d, const int* status, int* hstatus,
+                                cudaStream_t st) {
+  host_rows_kernel<false, T><<<rows_grid(d), 256, 0, st>>>(nullptr, host, src, nullptr, d, status, hstatus);
   return cudaGetLastError();
 }
 template cudaError_t launch_host_gather<double>(const double*, double*, const Dims&, cudaStream_t);
 template cudaError_t launch_host_gather<float>(const double*, float*, const Dims&, cudaStream_t);
-template cudaError_t launch_host_scatter<double>(const double*, double*, const Dims&, cudaStream_t);
-template cudaError_t launch_host_scatter<float>(const float*, double*, const Dims&, cudaStream_t);
+template cudaError_t launch_host_scatter<double>(const double*, double*, const Dims&, const int*, int*, cudaStream_t);
+template cudaError_t launch_host_scatter<float>(const float*, double*, const Dims&, const int*, int*, cudaStream_t);
 
 PlaneSched make_sched(const Dims& d, const StepTuning& tn, int gz) {
   PlaneSched S;

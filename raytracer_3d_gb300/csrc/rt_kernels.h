@@ -47,11 +47,12 @@ template <class T>
 cudaError_t launch_coeff(const Dims& d, const Background& bg, const Grid& g, const Phys& ph, const CoeffOut<T>& out,
                          double* scratch, int ring, double* rate, int* nlaunch, cudaStream_t st);
 // padded host array (pageable, read / written by the GPU directly) <-> the
-// unpadded device field
+// unpadded device field; the scatter also writes *status to the host int *hstatus
 template <class T>
 cudaError_t launch_host_gather(const double* host, T* dst, const Dims& d, cudaStream_t st);
 template <class T>
-cudaError_t launch_host_scatter(const T* src, double* host, const Dims& d, cudaStream_t st);
+cudaError_t launch_host_scatter(const T* src, double* host, const Dims& d, const int* status, int* hstatus,
+                                cudaStream_t st);
 cudaError_t launch_ucfl(const Dims& d, const Grid& g, double dt, const double* const* vel,
                         const double* const* vlo, double* const* uc, double* const* ucl,
                         cudaStream_t st);
