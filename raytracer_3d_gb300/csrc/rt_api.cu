@@ -54,6 +54,7 @@ struct rt_handle {
   SplitFluxes split{};          // flux fields of the fast binary64 step (allocated on selection)
   SplitFluxes slab{};           // flux scratch of the bit-exact step's slabs (allocated by the first such step)
   double* slab_mem = nullptr;
+  double* terms = nullptr;      // terms of the budget's wavenumber integrals, one slab (allocated by the first budget)
   int slab_state = 0;           // 0: not asked for yet, 1: there, -1: no memory for it
   double* mu = nullptr;         // fast binary64 step: 1 - dt*lambda per cell (allocated on selection)
   double* tab64 = nullptr;      // and its tables dt/d_a (offsets toff[0..5])
@@ -302,6 +303,19 @@ static bool slab_scratch(rt_handle* h) {
     p += (len[a] + 1) / 2 * 2;
   }
   h->slab_state = 1;
+  return true;
+}
+
+// scratch of the budget's wavenumber integrals (false: no memory)
+static bool budget_scratch(rt_handle* h) {
+  if (h->terms) return true;
+  const size_t n = (size_t)budget_terms(h->d) * sizeof(double);
+  if (cudaMalloc((void**)&h->terms, n) != cudaSuccess) {
+    cudaGetLastError();
+    h->terms = nullptr;
+    return false;
+  }
+  h->bytes += (long long)n;
   return true;
 }
 
@@ -1155,6 +1169,7 @@ int rt_destroy(rt_handle* h) {
   cudaFree(h->force);
   for (int a = 0; a < 6; a++) { cudaFree(h->split.f[a]); cudaFree(h->split.f0[a]); }
   cudaFree(h->slab_mem);
+  cudaFree(h->terms);
   cudaFree(h->mu);
   cudaFree(h->tab64);
   for (auto& kv : h->timers) {
@@ -1542,13 +1557,17 @@ int rt_diagnose(rt_handle* h, rt_budget* o, double* E_int, double* meanfl_int, d
   const Dims& d = h->d;
   const int prev = 1 - h->cur;  // state before the last step
   cudaError_t e;
-  if (h->p.precision == RT_FP64)
+  int nl = 4;
+  if (h->p.precision == RT_FP64 && d.ncell < (1ll << 31) && slab_scratch(h) && budget_scratch(h))
+    e = launch_budget_exact(make_step_args<double>(h, prev), (const double*)h->E[h->cur], h->slab, h->uc_holds == 0,
+                            h->terms, h->scratch, h->vol3, h->result, &nl, h->st);
+  else if (h->p.precision == RT_FP64)
     e = launch_diag<double>(make_step_args<double>(h, prev), (const double*)h->E[h->cur], h->scratch,
                             h->vol3, h->result, h->st);
   else
     e = launch_diag<float>(make_step_args<float>(h, prev), (const float*)h->E[h->cur], h->scratch,
                            h->vol3, h->result, h->st);
-  h->launches += 4;
+  h->launches += nl;
   if (e != cudaSuccess) return fail(h, RT_ERR_CUDA, "diagnose launch: %s", cudaGetErrorString(e));
   double r[DIAG_RESULT_NV];
   CUDA_TRY(h, cudaMemcpyAsync(r, h->result, sizeof(r), cudaMemcpyDeviceToHost, h->st));

@@ -322,12 +322,20 @@ struct Slab {
   int ax, s_ax;         // slab axis and its stride
   int ring;             // planes of the flux ring along the slab axis
   int q0;               // first entry of the slab in the face-0 plane of z
+  int c0, c1;           // values of the slab axis
 };
 
 __device__ __forceinline__ int ring_at(const Slab& L, int p, int c) {
   return p - c * L.s_ax + (c % L.ring) * L.s_ax;
 }
 
+// uCFL of a face, |v*dt/d| (superbee_fluxes.f90:19), where no cached one is at hand
+__device__ __forceinline__ double face_ucfl(const StepArgs<double>& A, int a, int f, double v) {
+  return fabs(div_rn(dmul(v, A.dt), A.g.d[a][pidx(f)]));
+}
+
+// CACHED: uc holds the uCFL (it holds the fast step's h otherwise)
+template <bool CACHED>
 __global__ void __launch_bounds__(256, 4) exact_flux_kernel(StepArgs<double> A, SplitFluxes F, CellGeom G, Slab L) {
   const Dims& d = A.d;
   const unsigned pu = L.base + blockIdx.x * blockDim.x + threadIdx.x;
@@ -343,11 +351,14 @@ __global__ void __launch_bounds__(256, 4) exact_flux_kernel(StepArgs<double> A, 
     const double Em1 = A.E[nb32(d, G, p, a, ca, -1, c[5])];
     const double Ep1 = A.E[nb32(d, G, p, a, ca, +1, c[5])];
     const double Ep2 = A.E[nb32(d, G, p, a, ca, +2, c[5])];
-    const double f = flux_exact(__ldcs(A.vel[a] + p), __ldcs(A.uc[a] + p), Em1, e0, Ep1, Ep2);
+    const double v = __ldcs(A.vel[a] + p);
+    const double u = CACHED ? __ldcs(A.uc[a] + p) : face_ucfl(A, a, ca + 1, v);
+    const double f = flux_exact(v, u, Em1, e0, Ep1, Ep2);
     F.f[a][a == L.ax ? ring_at(L, p, ca) : p - (int)L.base] = f;
     if (ca == 0 && !face0_is_copy(d, a)) {
       const int q = plane32(G, a, c);
-      F.f0[a][q - L.q0] = flux_exact(A.vlo[a][q], A.ucl[a][q], A.E[nb32(d, G, p, a, ca, -2, c[5])], Em1, e0, Ep1);
+      const double v0 = A.vlo[a][q], u0 = CACHED ? A.ucl[a][q] : face_ucfl(A, a, 0, v0);
+      F.f0[a][q - L.q0] = flux_exact(v0, u0, A.E[nb32(d, G, p, a, ca, -2, c[5])], Em1, e0, Ep1);
     }
   }
 }
@@ -486,22 +497,34 @@ cudaError_t launch_step_exact_small(const StepArgs<double>& A, int nsteps, int f
   return cudaLaunchCooperativeKernel((const void*)kernel, dim3(ctas), dim3((unsigned)threads), args, sm, st);
 }
 
+namespace {
+
+// values [c0, c0 + m) of axis ax
+Slab make_slab(const Dims& d, int ax, int m, int c0) {
+  const int count = c0 + m <= d.n[ax] ? m : d.n[ax] - c0;
+  Slab L;
+  L.base = (unsigned)(c0 * d.s[ax]);
+  L.end = (unsigned)((c0 + count) * d.s[ax]);
+  L.ax = ax;
+  L.s_ax = (int)d.s[ax];
+  L.ring = m == d.n[ax] ? m : m + 1;
+  L.q0 = ax == 2 ? 0 : (int)(c0 * (d.s[ax] / d.n[2]));
+  L.c0 = c0;
+  L.c1 = c0 + count;
+  return L;
+}
+
+}  // namespace
+
 cudaError_t launch_step_exact_slabs(const StepArgs<double>& A, const SplitFluxes& F, cudaStream_t st, int* nlaunch) {
   const Dims& d = A.d;
   const CellGeom G = make_cells(d);
   const int ax = slab_axis(d), m = exact_slab_planes(d);
   *nlaunch = 0;
   for (int c0 = 0; c0 < d.n[ax]; c0 += m) {
-    const int count = c0 + m <= d.n[ax] ? m : d.n[ax] - c0;
-    Slab L;
-    L.base = (unsigned)(c0 * d.s[ax]);
-    L.end = (unsigned)((c0 + count) * d.s[ax]);
-    L.ax = ax;
-    L.s_ax = (int)d.s[ax];
-    L.ring = m == d.n[ax] ? m : m + 1;
-    L.q0 = ax == 2 ? 0 : (int)(c0 * (d.s[ax] / d.n[2]));
+    const Slab L = make_slab(d, ax, m, c0);
     const unsigned blocks = (L.end - L.base + 255) / 256;
-    exact_flux_kernel<<<blocks, 256, 0, st>>>(A, F, G, L);
+    exact_flux_kernel<true><<<blocks, 256, 0, st>>>(A, F, G, L);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     exact_update_kernel<<<blocks, 256, 0, st>>>(A, F, G, L);
@@ -510,6 +533,288 @@ cudaError_t launch_step_exact_slabs(const StepArgs<double>& A, const SplitFluxes
     *nlaunch += 2;
   }
   return cudaSuccess;
+}
+
+// ---------------------------------------------------------------------------
+// energy budget (diagnose.f90:46-277) of the step from A.E to Ecur, over the
+// same slabs: the fluxes once per face, then
+//   budget_cells_kernel   per cell dE and meanfl as the update forms them, the
+//                         scalar sums and maxima, and the terms of E_int and
+//                         meanfl_int (products of the reference's order);
+//   budget_tail_kernel    the boundary-flux sums, and beside them the eight
+//                         wavenumber integrals of every spatial cell, each a
+//                         chain of additions in the reference's order.
+// The fluxes and cells are bound by the binary64 pipe (about 105 instructions
+// per cell).  A chain is bound by the 64 cycles that a binary64 instruction
+// takes a warp whatever its lanes do, so it adds and does nothing else that
+// could be done elsewhere.
+// ---------------------------------------------------------------------------
+namespace {
+
+constexpr int kBudgetBlocks = 8 * 152;
+
+// max of two non-negative doubles by their bits (NaN above all)
+__device__ __forceinline__ double max_bits(double a, double b) {
+  const unsigned long long x = (unsigned long long)__double_as_longlong(a), y = (unsigned long long)__double_as_longlong(b);
+  return x > y ? a : b;
+}
+
+__global__ void __launch_bounds__(256, 3) budget_cells_kernel(StepArgs<double> A, const double* __restrict__ Ecur,
+                                                              SplitFluxes F, CellGeom G, Slab L,
+                                                              double* __restrict__ te, double* __restrict__ tm,
+                                                              double* __restrict__ partial) {
+  __shared__ double red[8][DIAG_CELL_NV];
+  const Dims& d = A.d;
+  double acc[DIAG_CELL_NV];
+#pragma unroll
+  for (int k = 0; k < DIAG_CELL_NV; k++) acc[k] = 0.0;
+  for (unsigned pu = L.base + blockIdx.x * blockDim.x + threadIdx.x; pu < L.end; pu += gridDim.x * blockDim.x) {
+    const int p = (int)pu, q = p - (int)L.base;
+    int c[6];
+    cell_coords(G, pu, c);
+    const double e0 = A.E[p];
+    double dE = 0., w[6];
+#pragma unroll
+    for (int a = 0; a < 6; a++) {
+      const int ca = c[a];
+      w[a] = A.g.d[a][pidx(ca + 1)];
+      acc[3 + a] = max_bits(acc[3 + a], fabs(__ldcs(A.vel[a] + p)));
+      if (d.n[a] <= 1) continue;
+      const double fr = F.f[a][a == L.ax ? ring_at(L, p, ca) : q];
+      double fl;
+      if (ca > 0) {
+        fl = F.f[a][a == L.ax ? ring_at(L, p - L.s_ax, ca - 1) : q - G.s[a]];
+      } else {
+        const int q0 = plane32(G, a, c);
+        fl = face0_is_copy(d, a) ? dmul(A.vlo[a][q0], e0) : F.f0[a][q0 - L.q0];
+      }
+      dE = dsub(dE, div_rn(dsub(fr, fl), w[a]));
+    }
+    double mf = 0.;
+    if (d.n[0] > 1) mf = dmul(e0, __ldcs(A.lam[0] + p));
+    if (d.n[1] > 1) mf = dadd(mf, dmul(e0, __ldcs(A.lam[1] + p)));
+    if (d.n[2] > 1) mf = dadd(mf, dmul(e0, __ldcs(A.lam[2] + p)));
+    double vol = w[0];
+#pragma unroll
+    for (int a = 1; a < 6; a++) vol = dmul(vol, w[a]);
+    acc[0] = dadd(acc[0], dmul(dsub(dE, mf), vol));
+    acc[1] = dadd(acc[1], dmul(mf, vol));
+    const double ec = Ecur[p];
+    const Bits64 eb = split64(ec);
+    const long long ebits = (long long)(((uint64_t)eb.hi << 32) | eb.lo);
+    const double floor_e = ebits > __double_as_longlong(RT_LIT_1EM12) ? ec : RT_LIT_1EM12;   // diagnose.f90:56
+    acc[2] = max_bits(acc[2], div_rn(fabs(mf), floor_e));
+    te[q] = dmul(dmul(dmul(ec, w[4]), w[5]), w[3]);   // E*dlt*dmt*dkt, diagnose.f90:90
+    tm[q] = dmul(dmul(dmul(mf, w[3]), w[4]), w[5]);
+  }
+  // block partials in a fixed order: lanes, then warps; they add to those of
+  // the slabs before
+#pragma unroll
+  for (int k = 0; k < DIAG_CELL_NV; k++) {
+    double x = acc[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double y = __shfl_down_sync(0xffffffffu, x, o);
+      x = k < 2 ? dadd(x, y) : max_bits(x, y);
+    }
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][k] = x;
+  }
+  __syncthreads();
+  if (threadIdx.x < DIAG_CELL_NV) {
+    const int k = threadIdx.x;
+    double* out = partial + (long long)blockIdx.x * DIAG_CELL_NV + k;
+    double x = L.base == 0 ? red[0][k] : (k < 2 ? dadd(*out, red[0][k]) : max_bits(*out, red[0][k]));
+    for (int wi = 1; wi < 8; wi++) x = k < 2 ? dadd(x, red[wi][k]) : max_bits(x, red[wi][k]);
+    *out = x;
+  }
+}
+
+// flux through face 0 (hi = false) or face n of axis a at the boundary cell p
+template <int a>
+__device__ __forceinline__ double face_at(const StepArgs<double>& A, const SplitFluxes& F, const CellGeom& G,
+                                          const Slab& L, bool hi, int p, const int c[6]) {
+  if (hi) return F.f[a][a == L.ax ? ring_at(L, p, c[a]) : p - (int)L.base];
+  const int q0 = plane32(G, a, c);
+  return face0_is_copy(A.d, a) ? dmul(A.vlo[a][q0], A.E[p]) : F.f0[a][q0 - L.q0];
+}
+
+// a thread's share of the boundary sum through face 0 / n of axis a
+template <int a>
+__device__ __forceinline__ double plane_share(const StepArgs<double>& A, const SplitFluxes& F, const CellGeom& G,
+                                              const Slab& L, bool hi, unsigned blk, unsigned nblk) {
+  const Dims& d = A.d;
+  const int cb = hi ? d.n[a] - 1 : 0;
+  double acc = 0.0;
+  if (d.n[a] <= 1 || (a == L.ax && (cb < L.c0 || cb >= L.c1))) return acc;
+  // boundary cells of the slab: the slab's cells with axis a at cb
+  const unsigned cells = a == L.ax ? (unsigned)L.s_ax : (L.end - L.base) / (unsigned)d.n[a];
+  const unsigned s = (unsigned)G.s[a];
+  for (unsigned q = blk * blockDim.x + threadIdx.x; q < cells; q += nblk * blockDim.x) {
+    const unsigned p = a == L.ax ? (unsigned)cb * s + q
+                                 : L.base + (q / s) * (s * (unsigned)d.n[a]) + (unsigned)cb * s + q % s;
+    int c[6];
+    cell_coords(G, p, c);
+    double area = 0.0;
+    bool first = true;
+#pragma unroll
+    for (int b = 0; b < 6; b++) {
+      if (b == a) continue;
+      const double db = A.g.d[b][pidx(c[b] + 1)];
+      area = first ? db : dmul(area, db);
+      first = false;
+    }
+    acc = dadd(acc, dmul(face_at<a>(A, F, G, L, hi, (int)p, c), area));
+  }
+  return acc;
+}
+
+// block b of nblk of boundary `which` = 2*axis + (0: face 0, 1: face n);
+// partial layout [axis][block][2]
+__device__ __forceinline__ void budget_planes(const StepArgs<double>& A, const SplitFluxes& F, const CellGeom& G,
+                                              const Slab& L, int which, unsigned b, unsigned nblk, double* partial,
+                                              double red[4]) {
+  const int a = which >> 1;
+  const bool hi = which & 1;
+  double acc = a == 0   ? plane_share<0>(A, F, G, L, hi, b, nblk)
+               : a == 1 ? plane_share<1>(A, F, G, L, hi, b, nblk)
+               : a == 2 ? plane_share<2>(A, F, G, L, hi, b, nblk)
+               : a == 3 ? plane_share<3>(A, F, G, L, hi, b, nblk)
+               : a == 4 ? plane_share<4>(A, F, G, L, hi, b, nblk)
+                        : plane_share<5>(A, F, G, L, hi, b, nblk);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc = dadd(acc, __shfl_down_sync(0xffffffffu, acc, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double* out = partial + ((long long)a * nblk + b) * 2 + (hi ? 1 : 0);
+    double x = L.base == 0 ? 0.0 : *out;
+    for (int w = 0; w < 4; w++) x = dadd(x, red[w]);
+    *out = x;
+  }
+}
+
+// diss_{a}s / diss_{a}e of a spatial cell: the boundary fluxes over the two
+// other spectral axes, the slower one outside (diagnose.f90:186-277)
+template <int a>
+__device__ __forceinline__ double diss_chain(const StepArgs<double>& A, const SplitFluxes& F, const CellGeom& G,
+                                             const Slab& L, bool hi, int v3, double acc) {
+  const Dims& d = A.d;
+  const int cb = hi ? d.n[a] - 1 : 0;
+  if (d.n[a] <= 1 || (a == L.ax && (cb < L.c0 || cb >= L.c1))) return acc;
+  constexpr int b1 = a == 3 ? 4 : 3, b2 = a == 5 ? 4 : 5;
+  int c[6];
+  cell_coords(G, (unsigned)v3, c);
+  c[a] = cb;
+  const int lo1 = b1 == L.ax ? L.c0 : 0, hi1 = b1 == L.ax ? L.c1 : d.n[b1];
+  const int lo2 = b2 == L.ax ? L.c0 : 0, hi2 = b2 == L.ax ? L.c1 : d.n[b2];
+  for (int i2 = lo2; i2 < hi2; i2++) {
+    c[b2] = i2;
+    const double w2 = A.g.d[b2][pidx(i2 + 1)];
+#pragma unroll 4
+    for (int i1 = lo1; i1 < hi1; i1++) {
+      c[b1] = i1;
+      const int p = v3 + c[3] * G.s[3] + c[4] * G.s[4] + c[5] * G.s[5];
+      acc = dadd(acc, dmul(dmul(face_at<a>(A, F, G, L, hi, p, c), A.g.d[b1][pidx(i1 + 1)]), w2));
+    }
+  }
+  return acc;
+}
+
+// 32 spatial cells (group `g` of them) and the integral f: E_int, meanfl_int,
+// diss_ks, diss_ke, diss_ls, diss_le, diss_ms, diss_me; carried from slab to
+// slab in out
+__device__ __forceinline__ void budget_chain(const StepArgs<double>& A, const SplitFluxes& F, const CellGeom& G,
+                                             const Slab& L, const double* __restrict__ te,
+                                             const double* __restrict__ tm, unsigned g, int f, double* out) {
+  const unsigned nvol3 = (unsigned)A.d.nvol3;
+  const unsigned v3 = g * 32 + (threadIdx.x & 31);
+  if (v3 >= nvol3) return;
+  if (L.ax < 3 && (v3 < L.base || v3 >= L.end)) return;   // a slab of space holds whole spatial cells
+  const bool fresh = L.ax < 3 || L.base == 0;
+  double acc = fresh ? 0.0 : out[(long long)f * nvol3 + v3];
+  if (f < 2) {
+    const double* t = (f == 0 ? te : tm) + (L.ax < 3 ? v3 - L.base : v3);
+    const int n = L.ax < 3 ? 1 : (int)((L.end - L.base) / nvol3);
+    constexpr int U = 16;
+    int i = 0;
+    double x[U];
+    if (n >= U) {
+#pragma unroll
+      for (int k = 0; k < U; k++) x[k] = __ldcg(t + (long long)k * nvol3);
+      for (; i + 2 * U <= n; i += U) {
+        double y[U];
+#pragma unroll
+        for (int k = 0; k < U; k++) y[k] = __ldcg(t + (long long)(i + U + k) * nvol3);
+#pragma unroll
+        for (int k = 0; k < U; k++) acc = dadd(acc, x[k]);
+#pragma unroll
+        for (int k = 0; k < U; k++) x[k] = y[k];
+      }
+#pragma unroll
+      for (int k = 0; k < U; k++) acc = dadd(acc, x[k]);
+      i += U;
+    }
+    for (; i < n; i++) acc = dadd(acc, __ldcg(t + (long long)i * nvol3));
+  } else if (f < 4) {
+    acc = diss_chain<3>(A, F, G, L, f & 1, (int)v3, acc);
+  } else if (f < 6) {
+    acc = diss_chain<4>(A, F, G, L, f & 1, (int)v3, acc);
+  } else {
+    acc = diss_chain<5>(A, F, G, L, f & 1, (int)v3, acc);
+  }
+  out[(long long)f * nvol3 + v3] = acc;
+}
+
+// blocks [0, 2*groups): the chains of 32 spatial cells, four integrals each,
+// one a warp (the four schedulers' binary64 paths are separate: 76 cycles an
+// instruction for four warps, 64 for one, 128 for two on one scheduler); the
+// others the boundary sums, which fill the pipe beside them
+__global__ void __launch_bounds__(128) budget_tail_kernel(StepArgs<double> A, SplitFluxes F, CellGeom G, Slab L,
+                                                          const double* __restrict__ te, const double* __restrict__ tm,
+                                                          unsigned groups, unsigned nblk, double* vol3,
+                                                          double* partial) {
+  __shared__ double red[4];
+  const unsigned b = blockIdx.x;
+  if (b < 2 * groups)
+    budget_chain(A, F, G, L, te, tm, b >> 1, (int)((b & 1) + 2 * (threadIdx.x >> 5)), vol3);
+  else
+    budget_planes(A, F, G, L, (int)((b - 2 * groups) / nblk), (b - 2 * groups) % nblk, nblk, partial, red);
+}
+
+}  // namespace
+
+long long budget_terms(const Dims& d) { return 2 * exact_slab_planes(d) * d.s[slab_axis(d)]; }
+
+cudaError_t launch_budget_exact(const StepArgs<double>& A, const double* Ecur, const SplitFluxes& F, bool ucfl_cached,
+                                double* terms, double* scratch, double* vol3, double* result, int* nlaunch,
+                                cudaStream_t st) {
+  const Dims& d = A.d;
+  const CellGeom G = make_cells(d);
+  const int ax = slab_axis(d), m = exact_slab_planes(d);
+  const DiagSizes sizes = diag_sizes(d);
+  double* te = terms;
+  double* tm = terms + budget_terms(d) / 2;
+  const unsigned cb = (unsigned)std::min<long long>(kBudgetBlocks, (std::min<long long>(m * d.s[ax], d.ncell) + 255) / 256);
+  const unsigned pb = (unsigned)std::min<long long>(sizes.plane_blocks, (m * d.s[ax] + 1023) / 1024);
+  const unsigned groups = (unsigned)((d.nvol3 + 31) / 32);
+  double* pc = scratch;
+  double* pp = scratch + (long long)cb * DIAG_CELL_NV;
+  *nlaunch = 0;
+  cudaError_t e;
+  for (int c0 = 0; c0 < d.n[ax]; c0 += m) {
+    const Slab L = make_slab(d, ax, m, c0);
+    const unsigned blocks = (L.end - L.base + 255) / 256;
+    if (ucfl_cached) exact_flux_kernel<true><<<blocks, 256, 0, st>>>(A, F, G, L);
+    else exact_flux_kernel<false><<<blocks, 256, 0, st>>>(A, F, G, L);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    budget_cells_kernel<<<cb, 256, 0, st>>>(A, Ecur, F, G, L, te, tm, pc);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    budget_tail_kernel<<<2 * groups + 12 * pb, 128, 0, st>>>(A, F, G, L, te, tm, groups, pb, vol3, pp);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    *nlaunch += 3;
+  }
+  *nlaunch += 1;
+  return launch_diag_finish(pc, cb, pp, pb, result, st);
 }
 
 }  // namespace rt

@@ -325,43 +325,25 @@ __global__ void __launch_bounds__(128) diag_vol3_kernel(StepArgs<T> A, const T* 
   out[7 * d.nvol3 + v3] = me;
 }
 
-// final fixed-order reduction of the partials (one block)
-__global__ void diag_finish_kernel(const double* pc, long long ncb, const double* pp, long long npb,
-                                   double* out) {
+// final fixed-order reduction of the partials, one block per value: the cell
+// values, then 6 axes x {lo, hi}
+__global__ void __launch_bounds__(256) diag_finish_kernel(const double* pc, long long ncb, const double* pp,
+                                                          long long npb, double* out) {
   __shared__ double red[256];
-  // cell partials
-  for (int k = 0; k < DIAG_CELL_NV; k++) {
-    double acc = 0.0;
-    for (long long i = threadIdx.x; i < ncb; i += blockDim.x) {
-      const double x = pc[i * DIAG_CELL_NV + k];
-      acc = (k < 2) ? dadd(acc, x) : fmax2(acc, x);
-    }
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-      if (threadIdx.x < w)
-        red[threadIdx.x] = (k < 2) ? dadd(red[threadIdx.x], red[threadIdx.x + w])
-                                   : fmax2(red[threadIdx.x], red[threadIdx.x + w]);
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) out[k] = red[0];
+  const int k = blockIdx.x;
+  const bool sum = k < 2 || k >= DIAG_CELL_NV;
+  const double* src = k < DIAG_CELL_NV ? pc + k : pp + (long long)((k - DIAG_CELL_NV) / 2) * npb * 2 + (k - DIAG_CELL_NV) % 2;
+  const long long n = k < DIAG_CELL_NV ? ncb : npb, step = k < DIAG_CELL_NV ? DIAG_CELL_NV : 2;
+  double acc = 0.0;
+  for (long long i = threadIdx.x; i < n; i += blockDim.x) acc = sum ? dadd(acc, src[i * step]) : fmax2(acc, src[i * step]);
+  red[threadIdx.x] = acc;
+  __syncthreads();
+  for (int w = 128; w > 0; w >>= 1) {
+    if (threadIdx.x < w)
+      red[threadIdx.x] = sum ? dadd(red[threadIdx.x], red[threadIdx.x + w]) : fmax2(red[threadIdx.x], red[threadIdx.x + w]);
     __syncthreads();
   }
-  // plane partials: 6 axes x {lo, hi}
-  for (int k = 0; k < 12; k++) {
-    const int a = k / 2, side = k % 2;
-    double acc = 0.0;
-    for (long long i = threadIdx.x; i < npb; i += blockDim.x)
-      acc = dadd(acc, pp[((long long)a * npb + i) * 2 + side]);
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-      if (threadIdx.x < w) red[threadIdx.x] = dadd(red[threadIdx.x], red[threadIdx.x + w]);
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) out[DIAG_CELL_NV + k] = red[0];
-    __syncthreads();
-  }
+  if (threadIdx.x == 0) out[k] = red[0];
 }
 
 // ---------------------------------------------------------------------------
@@ -678,6 +660,12 @@ DiagSizes diag_sizes(const Dims& d) {
   return s;
 }
 
+cudaError_t launch_diag_finish(const double* pc, long long ncb, const double* pp, long long npb, double* result,
+                               cudaStream_t st) {
+  diag_finish_kernel<<<DIAG_RESULT_NV, 256, 0, st>>>(pc, ncb, pp, npb, result);
+  return cudaGetLastError();
+}
+
 template <class T>
 cudaError_t launch_diag(const StepArgs<T>& A, const T* Ecur, double* scratch, double* vol3,
                         double* result, cudaStream_t st) {
@@ -693,8 +681,7 @@ cudaError_t launch_diag(const StepArgs<T>& A, const T* Ecur, double* scratch, do
   diag_vol3_kernel<T><<<(unsigned)((A.d.nvol3 + 127) / 128), 128, 0, st>>>(A, Ecur, vol3);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  diag_finish_kernel<<<1, 256, 0, st>>>(pc, s.cell_blocks, pp, s.plane_blocks, result);
-  return cudaGetLastError();
+  return launch_diag_finish(pc, s.cell_blocks, pp, s.plane_blocks, result, st);
 }
 template cudaError_t launch_diag<double>(const StepArgs<double>&, const double*, double*, double*,
                                          double*, cudaStream_t);

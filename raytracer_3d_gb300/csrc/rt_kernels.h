@@ -178,6 +178,13 @@ long long exact_scratch(const Dims& d, int a);
 long long exact_scratch_z0(const Dims& d);
 cudaError_t launch_step_exact_small(const StepArgs<double>& A, int nsteps, int forcing, const double* F, double dz,
                                     unsigned* counter, cudaStream_t st);
+// energy budget of the step from A.E to Ecur by the same slabs: terms: scratch
+// of budget_terms(d) doubles; ucfl_cached: A.uc holds the uCFL; the other
+// arguments as launch_diag's
+long long budget_terms(const Dims& d);
+cudaError_t launch_budget_exact(const StepArgs<double>& A, const double* Ecur, const SplitFluxes& F, bool ucfl_cached,
+                                double* terms, double* scratch, double* vol3, double* result, int* nlaunch,
+                                cudaStream_t st);
 cudaError_t launch_step_exact_slabs(const StepArgs<double>& A, const SplitFluxes& F, cudaStream_t st, int* nlaunch);
 // fast binary64 step (rt_fast.cu): the flux fields of the two-pass step,
 // h = |v|/2*(1-|v dt/d|) per face (hr: right faces, hl: face-0 planes),
@@ -207,6 +214,9 @@ cudaError_t launch_forcing(T* E, const double* F, const T* zdot, const Dims& d, 
 template <class T>
 cudaError_t launch_tendency(const StepArgs<T>& A, double* dE, double* meanfl, cudaStream_t st);
 DiagSizes diag_sizes(const Dims& d);
+// the partials [block][DIAG_CELL_NV] and [axis][block][2] to the result vector
+cudaError_t launch_diag_finish(const double* pc, long long ncb, const double* pp, long long npb, double* result,
+                               cudaStream_t st);
 template <class T>
 cudaError_t launch_diag(const StepArgs<T>& A, const T* Ecur, double* scratch, double* vol3,
                         double* result, cudaStream_t st);
