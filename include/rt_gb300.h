@@ -196,14 +196,12 @@ int rt_get_tendency(rt_handle* h, double* dE, double* meanfl);
  *        packed f32x2 instructions and the next plane's operands prefetched
  *        into L2
  *   15 = binary64: as 2
- *   16 = binary64 fast: two passes without divisions (limiter slope selected
- *        exactly, update regrouped; its fields, 56 bytes per cell, are
- *        allocated by this call);
+ *   16 = binary64 fast: without divisions (limiter slope selected exactly,
+ *        update regrouped; its fields are allocated by this call: 58 bytes
+ *        per cell and rings of slopes, 0.9 GB at 32^6 cells);
  *        within a few units in the last place of the reference's result per
- *        step, NOT bit-identical to it.  band = m values per band of its
- *        spectral-plane order (1: natural order; a width that does not
- *        divide nm is reduced to the largest one that does); fields of
- *        2^31 cells or more are rejected (RT_ERR_CUDA on the step)
+ *        step, NOT bit-identical to it.  band and threads have no effect;
+ *        fields of 2^31 cells or more are rejected (RT_ERR_CUDA on the step)
  * Every other variant gives the same result: bit-identical to the
  * reference's arithmetic in binary64, and among themselves in binary32.
  * band: values per band of the plane schedule (default 8); threads: CTA

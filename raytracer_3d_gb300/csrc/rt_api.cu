@@ -51,14 +51,18 @@ struct rt_handle {
   double* force = nullptr;      // its interior 5D field (x,y,k,l,m)
   long long force_gen = 0;      // changes with every rt_set_forcing
   double dzt1 = 0.0;            // dzt(1), the bottom cell's spacing
-  SplitFluxes split{};          // flux fields of the fast binary64 step (allocated on selection)
+  SplitFluxes fastv{};          // fast binary64 step: V of the right faces and face-0 planes (allocated on selection)
+  double* psi_mem = nullptr;    // its slope rings
+  double* psi[7]{};             // by axis, and the reflected z face 0
+  unsigned short* signs = nullptr;  // velocity signs per cell
+  int uniform = 0;              // every axis has one spacing
   SplitFluxes slab{};           // flux scratch of the bit-exact step's slabs (allocated by the first such step)
   double* slab_mem = nullptr;
   double* terms = nullptr;      // terms of the budget's wavenumber integrals, one slab (allocated by the first budget)
   int slab_state = 0;           // 0: not asked for yet, 1: there, -1: no memory for it
-  double* mu = nullptr;         // fast binary64 step: 1 - dt*lambda per cell (allocated on selection)
-  double* tab64 = nullptr;      // and its tables dt/d_a (offsets toff[0..5])
-  int uc_holds = 0;             // uc/ucl hold 0: uCFL of the bit-exact kernels, 1: h of the fast step
+  double* nu = nullptr;         // a cell's factor in the fast step (allocated on selection)
+  double* tab64 = nullptr;      // and its tables 1/d_a (offsets toff[0..5])
+  int uc_holds = 0;             // uc/ucl hold 0: uCFL of the bit-exact kernels, 1: H of the fast step
   double* scratch = nullptr;    // reductions
   long long scratch_len = 0;
   double* coeff_mem = nullptr;  // small fields: scratch of rt_calc_parameter
@@ -252,8 +256,29 @@ static cudaError_t apply_forcing(rt_handle* h, int buf, cudaStream_t st) {
                                h->forcing, st);
 }
 
+static FastFields fast_fields(const rt_handle* h) {
+  FastFields C{};
+  for (int a = 0; a < 6; a++) {
+    C.vel[a] = (const double*)h->vel[a];
+    C.vlo[a] = (const double*)h->vlo[a];
+    C.V[a] = h->fastv.f[a];
+    C.V0[a] = h->fastv.f0[a];
+    C.H[a] = h->uc[a];
+    C.H0[a] = h->ucl[a];
+    C.psi[a] = h->psi[a];
+    C.mask[a] = (unsigned)(fast_ring(h->d, a) - 1);
+    C.inv_d[a] = h->tab64 + h->toff[a];
+  }
+  for (int c = 0; c < 3; c++) C.lam[c] = (const double*)h->lam[c];
+  C.nu = h->nu;
+  C.signs = h->signs;
+  C.uniform = h->uniform;
+  C.psi0 = h->psi[6];
+  return C;
+}
+
 // the per-face values in uc/ucl for the kind of binary64 step about to run:
-// uCFL for the bit-exact kernels (kind 0), h, mu and the tables for the fast
+// uCFL for the bit-exact kernels (kind 0), the cached fields of the fast
 // step (kind 1); recomputed only when the kind changes (or dt / the
 // coefficients did, which resets uc_holds)
 static cudaError_t ensure_uc(rt_handle* h, int kind) {
@@ -266,20 +291,15 @@ static cudaError_t ensure_uc(rt_handle* h, int kind) {
     e = launch_ucfl(h->d, make_grid(h), h->p.dt, vel, vlo, h->uc, h->ucl, h->st);
     h->launches += 6;
   } else {
-    const double* lam[3] = {(const double*)h->lam[0], (const double*)h->lam[1], (const double*)h->lam[2]};
-    e = launch_fast_prepare(h->d, make_grid(h), h->p.dt, vel, vlo, lam, h->uc, h->ucl, h->mu, h->tab64, h->toff,
-                            h->st);
-    h->launches += 7;
+    int nl = 0;
+    e = launch_fast_prepare(h->d, make_grid(h), h->p.dt, fast_fields(h), h->tab64, h->toff, &nl, h->st);
+    h->launches += nl;
   }
   if (e == cudaSuccess) h->uc_holds = kind;
   return e;
 }
 
-static bool fast_ready(const rt_handle* h) {
-  bool split = false;
-  for (int a = 0; a < 6; a++) split = split || h->split.f[a] != nullptr;
-  return split && h->mu && h->tab64;
-}
+static bool fast_ready(const rt_handle* h) { return h->psi_mem && h->nu && h->tab64 && h->signs; }
 
 // scratch of the bit-exact step's slabs, one allocation; false when the
 // memory is not there (the handle then keeps the fused kernels, which need none)
@@ -333,10 +353,7 @@ static cudaError_t step_once(rt_handle* h, int src, int* nlaunch) {
     if (h->tune.variant == RT_VARIANT_FAST && fast_ready(h)) {
       cudaError_t e = ensure_uc(h, 1);
       if (e != cudaSuccess) return e;
-      FastTab T;
-      for (int a = 0; a < 6; a++) T.c[a] = h->tab64 + h->toff[a];
-      *nlaunch = 2;
-      return launch_step_fast(make_step_args<double>(h, src), h->split, h->mu, T, h->tune.band, h->st);
+      return launch_step_fast(h->d, fast_fields(h), (const double*)h->E[src], (double*)h->E[1 - src], nlaunch, h->st);
     }
     cudaError_t e = ensure_uc(h, 0);
     if (e != cudaSuccess) return e;
@@ -353,22 +370,32 @@ static cudaError_t step_once(rt_handle* h, int src, int* nlaunch) {
   return launch_step<float>(make_step_args<float>(h, src), h->tune, h->st);
 }
 
-// flux fields of the fast binary64 step, for the axes with n > 1
-static int ensure_split(rt_handle* h) {
-  const Dims& d = h->d;
-  for (int a = 0; a < 6; a++) {
-    if (d.n[a] <= 1 || h->split.f[a]) continue;
-    int rc = dev_alloc(h, (void**)&h->split.f[a], (size_t)d.ncell * sizeof(double));
-    if (!rc) rc = dev_alloc(h, (void**)&h->split.f0[a], (size_t)(d.ncell / d.n[a]) * sizeof(double));
-    if (rc) return rc;
-  }
-  return RT_OK;
-}
-
-// fast binary64 step: mu and the tables (its flux fields are the two-pass step's)
+// fast binary64 step: V for the axes with n > 1, the slope rings, nu, the
+// signs and the tables; a field with no such axis keeps the bit-exact step,
+// and so does one the step rejects
 static int ensure_fast(rt_handle* h) {
-  int rc = ensure_split(h);
-  if (!rc && !h->mu) rc = dev_alloc(h, (void**)&h->mu, (size_t)h->d.ncell * sizeof(double));
+  const Dims& d = h->d;
+  int rc = RT_OK;
+  long long ring = 0;
+  for (int a = 0; a < 6 && !rc; a++) {
+    if (d.n[a] <= 1) continue;
+    ring += fast_ring(d, a);
+    if (!h->fastv.f[a]) rc = dev_alloc(h, (void**)&h->fastv.f[a], (size_t)d.ncell * sizeof(double));
+    if (!rc && !h->fastv.f0[a])
+      rc = dev_alloc(h, (void**)&h->fastv.f0[a], (size_t)(d.ncell / d.n[a]) * sizeof(double));
+  }
+  if (d.n[2] > 1 && d.lower_refl) ring += fast_ring(d, 2);
+  if (!rc && ring && !h->psi_mem) {
+    rc = dev_alloc(h, (void**)&h->psi_mem, (size_t)ring * sizeof(double));
+    double* p = h->psi_mem;
+    for (int a = 0; a < 7 && !rc; a++) {
+      const long long len = a < 6 ? fast_ring(d, a) : (d.lower_refl ? fast_ring(d, 2) : 0);
+      h->psi[a] = len ? p : nullptr;
+      p += len;
+    }
+  }
+  if (!rc && !h->nu) rc = dev_alloc(h, (void**)&h->nu, (size_t)d.ncell * sizeof(double));
+  if (!rc && !h->signs) rc = dev_alloc(h, (void**)&h->signs, (size_t)d.ncell * sizeof(unsigned short));
   if (!rc && !h->tab64) rc = dev_alloc(h, (void**)&h->tab64, (size_t)h->toff[6] * sizeof(double));
   return rc;
 }
@@ -1167,10 +1194,12 @@ int rt_destroy(rt_handle* h) {
   cudaFree(h->status);
   cudaFree(h->seed);
   cudaFree(h->force);
-  for (int a = 0; a < 6; a++) { cudaFree(h->split.f[a]); cudaFree(h->split.f0[a]); }
+  for (int a = 0; a < 6; a++) { cudaFree(h->fastv.f[a]); cudaFree(h->fastv.f0[a]); }
+  cudaFree(h->psi_mem);
+  cudaFree(h->signs);
   cudaFree(h->slab_mem);
   cudaFree(h->terms);
-  cudaFree(h->mu);
+  cudaFree(h->nu);
   cudaFree(h->tab64);
   for (auto& kv : h->timers) {
     if (kv.second.open) cudaEventDestroy(kv.second.open);
@@ -1202,6 +1231,10 @@ int rt_set_grid(rt_handle* h, const double* dxt, const double* dyt, const double
     CUDA_TRY(h, cudaMemcpy(h->grid + h->goff[k], src[k], n * sizeof(double), cudaMemcpyHostToDevice));
   }
   h->dzt1 = dzt[pidx(1)];
+  h->uniform = 1;
+  for (int a = 0; a < 6; a++)
+    for (int f = 1; f <= h->d.n[a]; f++)   // faces 0..n
+      if (src[a][pidx(f)] != src[a][pidx(0)]) h->uniform = 0;
   int rc = upload_tab32(h);
   if (rc) return rc;
   h->have_grid = true;

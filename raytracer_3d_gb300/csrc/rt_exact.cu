@@ -22,63 +22,14 @@
 #include <algorithm>
 
 #include "../../include/rt_gb300.h"
+#include "rt_cells.cuh"
 #include "rt_exact.cuh"
-#include "rt_fast.cuh"
 #include "rt_kernels.h"
 #include "rt_step.cuh"
 
 namespace rt {
 
 namespace {
-
-// 32-bit index geometry (fields of 2^31 cells and more keep the other kernels)
-struct CellGeom {
-  unsigned ncell;
-  int s[6];
-  int ps[6][6];
-  DivU32 n[5];     // divisors of the coordinates, x..l
-};
-
-CellGeom make_cells(const Dims& d) {
-  CellGeom G;
-  G.ncell = (unsigned)d.ncell;
-  for (int a = 0; a < 6; a++) {
-    G.s[a] = (int)d.s[a];
-    for (int b = 0; b < 6; b++) G.ps[a][b] = (int)d.ps[a][b];
-    if (a < 5) G.n[a] = make_div((unsigned)d.n[a]);
-  }
-  return G;
-}
-
-__device__ __forceinline__ void cell_coords(const CellGeom& G, unsigned p, int c[6]) {
-  unsigned r = p;
-#pragma unroll
-  for (int a = 0; a < 5; a++) {
-    const unsigned q = G.n[a].div(r);
-    c[a] = (int)(r - q * G.n[a].d);
-    r = q;
-  }
-  c[5] = (int)r;
-}
-
-// nb_index and plane_index in 32-bit arithmetic
-__device__ __forceinline__ int nb32(const Dims& d, const CellGeom& G, int p, int a, int c, int off, int cm) {
-  int flip = 0;
-  const int c2 = map_coord(d, a, c + off, flip);
-  int q = p + (c2 - c) * G.s[a];
-  if (flip) q += ((d.n[5] - 1 - cm) - cm) * G.s[5];
-  return q;
-}
-__device__ __forceinline__ int plane32(const CellGeom& G, int a, const int c[6]) {
-  int q = 0;
-#pragma unroll
-  for (int b = 0; b < 6; b++) q += c[b] * G.ps[a][b];
-  return q;
-}
-
-// face 0 of an axis whose lower ghosts copy the edge cell: Rj = 0 and the
-// flux is v*(E0+E0)*0.5 = v*E0 exactly
-__device__ __forceinline__ bool face0_is_copy(const Dims& d, int a) { return a != 2 || !d.lower_refl; }
 
 // dE - meanfl and the update, integrate.f90:202-262
 __device__ __forceinline__ double exact_update(const StepArgs<double>& A, int p, double e0, double dE) {

@@ -73,7 +73,7 @@ cudaError_t launch_ucfl(const Dims& d, const Grid& g, double dt, const double* c
 #define RT_VARIANT_W2Q 18     // the same with the cell-pair arithmetic on packed f32x2 instructions and
                               // the next plane's operands prefetched into L2 (the binary32 production step)
 #define RT_VARIANT_SPLIT 15   // binary64: every face flux once, two passes (rt_exact.cu)
-#define RT_VARIANT_FAST 16    // binary64: two passes without divisions (rt_fast.cu), within 1e-12 of the reference
+#define RT_VARIANT_FAST 16    // binary64: without divisions, slopes on the integer pipes (rt_fast.cu), within 1e-12 of the reference
 struct StepTuning {
   int variant = RT_VARIANT_TMA;
   int band = 8;       // values per band of the plane schedule
@@ -186,20 +186,32 @@ cudaError_t launch_budget_exact(const StepArgs<double>& A, const double* Ecur, c
                                 double* terms, double* scratch, double* vol3, double* result, int* nlaunch,
                                 cudaStream_t st);
 cudaError_t launch_step_exact_slabs(const StepArgs<double>& A, const SplitFluxes& F, cudaStream_t st, int* nlaunch);
-// fast binary64 step (rt_fast.cu): the flux fields of the two-pass step,
-// h = |v|/2*(1-|v dt/d|) per face (hr: right faces, hl: face-0 planes),
-// mu = 1 - dt*lambda per cell and the per-axis tables c[a] = dt/d_a on the
-// padded index range
-struct FastTab {
-  const double* c[6];
+// fast binary64 step (rt_fast.cu).  V, H per face (V0, H0: face-0 planes, the
+// layout of vlo), nu and the velocity signs per cell, 1/d per axis; psi: rings
+// of fast_ring(d, a) doubles (mask: less one), psi0: as many as psi[2], with
+// the lower reflection only; uniform: every
+// axis has one spacing
+struct FastFields {
+  const double* vel[6];
+  const double* vlo[6];
+  const double* lam[3];
+  double* V[6];
+  double* V0[6];
+  double* H[6];
+  double* H0[6];
+  double* nu;
+  unsigned short* signs;
+  double* psi[6];
+  double* psi0;
+  unsigned mask[6];
+  const double* inv_d[6];
+  int uniform;
 };
-cudaError_t launch_fast_prepare(const Dims& d, const Grid& g, double dt, const double* const* vel,
-                                const double* const* vlo, const double* const* lam, double* const* hr,
-                                double* const* hl, double* mu, double* tab, const long long* toff,
-                                cudaStream_t st);
-// band: m values per band of the spectral-plane order (1: natural order)
-cudaError_t launch_step_fast(const StepArgs<double>& A, const SplitFluxes& F, const double* mu, const FastTab& T,
-                             int band, cudaStream_t st);
+long long fast_ring(const Dims& d, int a);
+cudaError_t launch_fast_prepare(const Dims& d, const Grid& g, double dt, const FastFields& C, double* tab,
+                                const long long* toff, int* nlaunch, cudaStream_t st);
+cudaError_t launch_step_fast(const Dims& d, const FastFields& C, const double* E, double* Enew, int* nlaunch,
+                             cudaStream_t st);
 // failure-detection self-test of the bounded waits (rt_persist.cu): one CTA
 // whose waits cannot complete; raises *status, leaves *completed at 0
 cudaError_t launch_wait_probe(int* status, int* completed, cudaStream_t st);
