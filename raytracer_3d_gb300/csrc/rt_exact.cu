@@ -11,14 +11,18 @@
 //
 // Both give the bits of the other binary64 kernels and of the oracle.
 //
-// The bound is the binary64 pipe: 10 instructions per face flux, two per
-// axis in the divergence and eight in the update, 80 per cell with six axes
-// in the two passes (290 with the divisions on that pipe).  32x32x32x12^3
-// measured 9.46 ms per step, 5.98 G cells/s and 478 G binary64
-// instructions/s, 90% of the measured rate; the TMA plane kernel took 39.9
+// The bound is the binary64 pipe: 7 instructions per face flux (10 where
+// values next to each other differ by more than 2^8), two per axis in the
+// divergence and seven in the update, 61 per cell with six axes in the two
+// passes (290 with the divisions on that pipe).  32x32x32x12^3 measured 7.65
+// ms per step, 7.4 G cells/s and 451 G binary64 instructions/s, 85% of the
+// measured rate (9.45 ms with 10 per flux); the TMA plane kernel took 39.9
 // ms, and a CTA of 512 threads per x-y plane 280 us for a 40x120 column
-// (one launch here: 8.2 us), 6.3 ms for a 10x20x60x60 section (97 us) and
-// 8.7 ms for 8x8x16x16^3 (0.74 ms).
+// (one launch here: 8.2 us), 6.3 ms for a 10x20x60x60 section (83 us) and
+// 8.7 ms for 8x8x16x16^3 (0.59 ms).  The integer work (340 instructions per
+// flux) wants many warps to hide behind: 32 registers and 8 resident CTAs
+// with some spilling measured 7.65 ms, 40 and 6 CTAs 7.90, 48 and 5 CTAs
+// 8.15, 52 and 4 CTAs 8.40.
 #include <algorithm>
 
 #include "../../include/rt_gb300.h"
@@ -285,12 +289,19 @@ __device__ __forceinline__ double face_ucfl(const StepArgs<double>& A, int a, in
   return fabs(div_rn(dmul(v, A.dt), A.g.d[a][pidx(f)]));
 }
 
+// 0 - q, on the integer pipes
+__device__ __forceinline__ double zero_minus(double q) {
+  const Bits64 b = split64(q);
+  return __hiloint2double((int)(is_zero(b) ? 0u : b.hi ^ 0x80000000u), (int)b.lo);
+}
+
 // CACHED: uc holds the uCFL (it holds the fast step's h otherwise)
 template <bool CACHED>
-__global__ void __launch_bounds__(256, 4) exact_flux_kernel(StepArgs<double> A, SplitFluxes F, CellGeom G, Slab L) {
+__global__ void __launch_bounds__(256, 8) exact_flux_kernel(StepArgs<double> A, SplitFluxes F, CellGeom G, Slab L) {
   const Dims& d = A.d;
-  const unsigned pu = L.base + blockIdx.x * blockDim.x + threadIdx.x;
-  if (pu >= L.end) return;
+  unsigned pu = L.base + blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = pu < L.end;
+  if (!valid) pu = L.end - 1;   // whole warps vote below
   const int p = (int)pu;
   int c[6];
   cell_coords(G, pu, c);
@@ -299,22 +310,25 @@ __global__ void __launch_bounds__(256, 4) exact_flux_kernel(StepArgs<double> A, 
   for (int a = 0; a < 6; a++) {
     if (d.n[a] <= 1) continue;
     const int ca = c[a];
-    const double Em1 = A.E[nb32(d, G, p, a, ca, -1, c[5])];
-    const double Ep1 = A.E[nb32(d, G, p, a, ca, +1, c[5])];
-    const double Ep2 = A.E[nb32(d, G, p, a, ca, +2, c[5])];
     const double v = __ldcs(A.vel[a] + p);
     const double u = CACHED ? __ldcs(A.uc[a] + p) : face_ucfl(A, a, ca + 1, v);
-    const double f = flux_exact(v, u, Em1, e0, Ep1, Ep2);
-    F.f[a][a == L.ax ? ring_at(L, p, ca) : p - (int)L.base] = f;
-    if (ca == 0 && !face0_is_copy(d, a)) {
+    const bool pos = f64_pos(v);
+    const double Ep1 = A.E[nb32(d, G, p, a, ca, +1, c[5])];
+    const double w = A.E[nb32(d, G, p, a, ca, pos ? -1 : +2, c[5])];
+    double f;
+    if (__all_sync(0xffffffffu, flux_is_near(v, u, e0, Ep1, w))) f = flux_near(v, u, e0, Ep1, w, pos);
+    else f = flux_exact(v, u, w, e0, Ep1, w);
+    if (valid) F.f[a][a == L.ax ? ring_at(L, p, ca) : p - (int)L.base] = f;
+    if (ca == 0 && valid && !face0_is_copy(d, a)) {
       const int q = plane32(G, a, c);
       const double v0 = A.vlo[a][q], u0 = CACHED ? A.ucl[a][q] : face_ucfl(A, a, 0, v0);
-      F.f0[a][q - L.q0] = flux_exact(v0, u0, A.E[nb32(d, G, p, a, ca, -2, c[5])], Em1, e0, Ep1);
+      F.f0[a][q - L.q0] = flux_exact(v0, u0, A.E[nb32(d, G, p, a, ca, -2, c[5])],
+                                     A.E[nb32(d, G, p, a, ca, -1, c[5])], e0, Ep1);
     }
   }
 }
 
-__global__ void __launch_bounds__(256, 4) exact_update_kernel(StepArgs<double> A, SplitFluxes F, CellGeom G, Slab L) {
+__global__ void __launch_bounds__(256, 8) exact_update_kernel(StepArgs<double> A, SplitFluxes F, CellGeom G, Slab L) {
   const Dims& d = A.d;
   const unsigned pu = L.base + blockIdx.x * blockDim.x + threadIdx.x;
   if (pu >= L.end) return;
@@ -323,6 +337,7 @@ __global__ void __launch_bounds__(256, 4) exact_update_kernel(StepArgs<double> A
   cell_coords(G, pu, c);
   const double e0 = A.E[p];
   double dE = 0.;
+  bool first = true;
 #pragma unroll
   for (int a = 0; a < 6; a++) {
     if (d.n[a] <= 1) continue;
@@ -335,7 +350,9 @@ __global__ void __launch_bounds__(256, 4) exact_update_kernel(StepArgs<double> A
       const int q0 = plane32(G, a, c);
       fl = face0_is_copy(d, a) ? dmul(A.vlo[a][q0], e0) : F.f0[a][q0 - L.q0];
     }
-    dE = dsub(dE, div_rn(dsub(fr, fl), A.g.d[a][pidx(ca + 1)]));
+    const double quo = div_rn(dsub(fr, fl), A.g.d[a][pidx(ca + 1)]);
+    dE = first ? zero_minus(quo) : dsub(dE, quo);
+    first = false;
   }
   __stcs(A.Enew + p, exact_update(A, p, e0, dE));
 }

@@ -14,13 +14,13 @@ from harness import ROOT, configs
 SRC = os.path.join(ROOT, "tests", "native", "exact_div_check.cu")
 
 
-def _check(tmp_path, *args, flags=()):
+def _check(tmp_path, *args, flags=(), src=SRC):
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(nvcc):
         pytest.skip("nvcc not found")
     exe = str(tmp_path / "exact_div_check")
     subprocess.run([nvcc, "-gencode", "arch=compute_103a,code=sm_103a", "-O2", "-std=c++17", *flags,
-                    "-I" + os.path.join(ROOT, "raytracer_3d_gb300", "csrc"), "-o", exe, SRC], check=True)
+                    "-I" + os.path.join(ROOT, "raytracer_3d_gb300", "csrc"), "-o", exe, src], check=True)
     r = subprocess.run([exe, *args], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
 
@@ -99,3 +99,34 @@ def test_many_steps_in_one_launch(n, forcing, walls):
     for E, b in got[1:]:
         assert np.array_equal(E, got[0][0])
         assert all(np.array_equal(x, y) for x, y in zip(b, got[0][1]))
+
+
+@pytest.mark.gpu
+def test_integer_differences_on_the_gpu(tmp_path):
+    _check(tmp_path, src=os.path.join(ROOT, "tests", "native", "flux_near_check.cu"))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -262])   # the second: next to the end of the integer range
+@pytest.mark.parametrize("n", [(16, 16, 64, 2, 70, 1), (15, 7, 12, 10, 12, 16)])
+def test_near_and_far_values_equal_the_cell_kernel(n, scale):
+    """most warps take the integer differences, those around the rough and the zero cells do not"""
+    import __graft_entry__ as g
+    g.build()
+    rng = np.random.default_rng(6)
+    exp = configs.shear_mini(n=n)
+    exp.fixed = (1e-3, 0.0, 1e-2)
+    sl = (slice(2, -2),) * 6
+    E0 = scale * (1 + 3 * rng.random(n))
+    E0[:, :, n[2] // 2, 0] *= rng.random(n)[:, :, n[2] // 2, 0] ** 20
+    E0[0, 0, 0] = 0.0
+    got = []
+    for variant in ("cell", "split"):
+        m = configs.build_model(exp, "fp64")
+        m.E[sl] = E0
+        m.set_state()
+        m.set_tuning(variant, 8, 256)
+        m.integrate(3)
+        got.append(m.get_state()[sl].copy())
+        m.close()
+    assert np.array_equal(got[0].view(np.uint64), got[1].view(np.uint64))
