@@ -9,22 +9,14 @@ namespace rt {
 
 namespace {
 
-// Resident CTAs per SM the walk is compiled for.  V = 4: a thread's 28 slots
-// are 56 KB per CTA and it wants 168 registers; 32x32x32x12x16x12 measured
-// 93.4 G cells/s at 3 CTAs, 90.5 at 4 (128 registers, spilling).  V = 2: 53.8
-// at 6, 52.0 at 5, 51.1 at 7 (30x18x20x14x10x12).  V = 1: 44.3 at 5, 37.4 at
-// 6 (15x9x21x8x16x10).
-constexpr int resident(int V) { return V == 4 ? 3 : (V == 2 ? 6 : 5); }
-
 template <int V>
-__global__ void __launch_bounds__(RT_MARCH_THREADS, resident(V)) march_kernel(const __grid_constant__ MarchArgs A) {
+__global__ void __launch_bounds__(RT_MARCH_THREADS, 1) march_kernel(const __grid_constant__ MarchArgs A) {
   march_cta<V>(A, blockIdx.x);
 }
 
 // V = 0: members of several widths
 template <int V>
-__global__ void __launch_bounds__(RT_MARCH_THREADS, resident(V ? V : 4))
-    march_batch_kernel(const __grid_constant__ MarchBatch B) {
+__global__ void __launch_bounds__(RT_MARCH_THREADS, 1) march_batch_kernel(const __grid_constant__ MarchBatch B) {
   int lo = 0, hi = B.nmem;   // first[lo] <= blockIdx.x < first[hi]
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;

@@ -11,15 +11,22 @@
 // slots of shared memory that it alone uses, so no barrier is needed and any
 // extents do: a field of odd or small planes runs like a large one.
 //
-// What bounds it: no pipe is full.  At 32x32x16x12x16x12 ncu counts 244
-// thread-instructions per cell (the z march, rt_step7.cuh: 346), issue slots
-// 59% and the ALU pipe (selects, minima, sign logic) 56% busy, DRAM 43 bytes
-// per cell (36 algorithmic), 12 warps per SM.  Loads straight into registers
-// left issue at 35% (61 G cells/s); the slots brought 93, the three-input
-// minimum 95.  Steps measured: 32^6 11.2 ms, 96 G cells/s (z march 15.9 ms);
-// 32x32x32x12x16x12 0.80 ms (1.27); 24x24x24x12x12x16 0.34 (0.87, TMA planes
-// 3.0); 30x18x20x14x10x12 0.32 (0.55, TMA planes 1.69); ensemble of ten
-// members, 110 M cells, 1.4 ms (3.6 in the two staged classes).
+// A part of the loop waits for its own copies only (one group of copies per
+// part, the six younger ones still under way), so each has a whole step of
+// the walk to arrive; one group for all, waited for right after its last
+// copy was issued, cost 12% (94 against 107 G cells/s).  Registers matter more
+// than resident warps: compiled without a lower bound on the CTAs per SM
+// (154, 116 and 96 registers; 12 to 20 warps) the widths V = 4, 2, 1 run at
+// 111.7, 83.5 and 47.9 G cells/s, with bounds of 3, 6 and 5 at 107.2, 64.9
+// and 44.1.  (V = 4 on rows that 4 does not divide, in copies of 8 or 4 bytes:
+// 50 and 29, L1 wavefronts.)
+//
+// What bounds it: 32x32x32x12x16x12 has the issue slots 66% and the ALU pipe
+// (selects, minima, sign logic) 62% busy, DRAM 67% at 50 bytes per cell (36
+// algorithmic).  Loads straight into registers left issue at 35% (61 G
+// cells/s).  Steps measured: 32^6 9.85 ms, 109 G cells/s (z march 15.9 ms);
+// 32x32x32x12x16x12 0.68 ms (1.27); 24x24x24x12x12x16 0.29 (0.87, TMA planes
+// 3.0); 30x18x20x14x10x12 0.22 (0.55, TMA planes 1.69).
 // The boundary maps are offsets fixed for the walk (a ghost that copies the
 // edge cell makes the difference zero and the flux v*E exactly), the face-0
 // velocities another base pointer.  Arithmetic per face and cell is that of
@@ -282,7 +289,7 @@ __device__ __forceinline__ void march_cta(const MarchArgs& A, unsigned item) {
   const int y = (int)(row - (unsigned)z * A.ny.d);
   const int k0 = (int)seg * A.klen, k1 = k0 + A.klen < nk ? k0 + A.klen : nk;
   const int sl = (int)nvol3 * nk, sm = sl * nl;
-  unsigned p = (unsigned)(m * nl + l) * (unsigned)sl + (unsigned)k0 * nvol3 + vec * V;
+  unsigned p = (unsigned)(m * nl + l) * (unsigned)sl + (unsigned)k0 * nvol3 + row * (unsigned)nx + (unsigned)x0;
   const unsigned kstep = nvol3 * 4u;
 
   unsigned oy[4], oz[4], ol[4], om[4];
@@ -333,23 +340,29 @@ __device__ __forceinline__ void march_cta(const MarchArgs& A, unsigned item) {
   unsigned pb = p * 4u;
   Vec<V> Ec = ldv<V>(A.E, pb), E1 = Ec, Dm = Ec, D0 = Ec, fk = Ec;   // E(k), E(k+1), D(k-1/2), D(k+1/2), left k flux
   // slots: 0 E(k+2); 1-4 y, 5-8 z, 9-12 l, 13-16 m neighbours; 17-22 right, 23-26 left velocities; 27 rate
-  if (ak) slot_fill<V>(slot0, A.E, k0 + 2 < nk ? pb + 2u * kstep : (k0 + 1 < nk ? pb + kstep : pb));
+  // one group of copies per part of the loop below, in its order
+  const auto commit = [] { asm volatile("cp.async.commit_group;"); };
+  const auto fill4 = [&](int first, const unsigned o[4]) {
 #pragma unroll
-  for (int j = 0; j < 4; j++) {
-    if (ay) slot_fill<V>(slot0 + (1 + j) * SS, A.E, pb + oy[j]);
-    if (az) slot_fill<V>(slot0 + (5 + j) * SS, A.E, pb + oz[j]);
-    if (al) slot_fill<V>(slot0 + (9 + j) * SS, A.E, pb + ol[j]);
-    if (am) slot_fill<V>(slot0 + (13 + j) * SS, A.E, pb + om[j]);
+    for (int j = 0; j < 4; j++) slot_fill<V>(slot0 + (first + j) * SS, A.E, pb + o[j]);
+  };
+  if (ax) slot_fill<V>(slot0 + 17 * SS, A.vel[0], pb);
+  commit();
+  if (ay) fill4(1, oy), slot_fill<V>(slot0 + 18 * SS, A.vel[1], pb), slot_fill<V>(slot0 + 23 * SS, lp[1], 0u);
+  commit();
+  if (az) fill4(5, oz), slot_fill<V>(slot0 + 19 * SS, A.vel[2], pb), slot_fill<V>(slot0 + 24 * SS, lp[2], 0u);
+  commit();
+  if (ak) {
+    slot_fill<V>(slot0, A.E, k0 + 2 < nk ? pb + 2u * kstep : (k0 + 1 < nk ? pb + kstep : pb));
+    slot_fill<V>(slot0 + 20 * SS, A.vel[3], pb);
   }
-#pragma unroll
-  for (int a = 0; a < 6; a++)
-    if (A.n[a] > 1) slot_fill<V>(slot0 + (17 + a) * SS, A.vel[a], pb);
-  if (ay) slot_fill<V>(slot0 + 23 * SS, lp[1], 0u);
-  if (az) slot_fill<V>(slot0 + 24 * SS, lp[2], 0u);
-  if (al) slot_fill<V>(slot0 + 25 * SS, lp[4], 0u);
-  if (am) slot_fill<V>(slot0 + 26 * SS, lp[5], 0u);
+  commit();
+  if (al) fill4(9, ol), slot_fill<V>(slot0 + 21 * SS, A.vel[4], pb), slot_fill<V>(slot0 + 25 * SS, lp[4], 0u);
+  commit();
+  if (am) fill4(13, om), slot_fill<V>(slot0 + 22 * SS, A.vel[5], pb), slot_fill<V>(slot0 + 26 * SS, lp[5], 0u);
+  commit();
   slot_fill<V>(slot0 + 27 * SS, A.lam, pb);
-  asm volatile("cp.async.commit_group;");
+  commit();
   float X0 = 0.f, X1 = 0.f, X2 = 0.f, X3 = 0.f, vxl = 0.f;   // E beside the row's part and its left x velocity
   if (ax) {
     X1 = ld1(A.E, inl ? pb - 4u : pb);
@@ -370,12 +383,12 @@ __device__ __forceinline__ void march_cta(const MarchArgs& A, unsigned item) {
   for (int k = k0; k < k1; k++) {
     const bool more = k + 1 < k1;
     const unsigned pn = pb + kstep;
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    // the part's copies of a k ago are there: six groups are younger
+    const auto filled = [] { asm volatile("cp.async.wait_group 6;" ::: "memory"); };
     Vec<V> E2 = Ec;
-    if (ak) {
-      E2 = slot_take<V>(slot0);
-      if (more) slot_fill<V>(slot0, A.E, k + 3 < nk ? pn + 2u * kstep : (k + 2 < nk ? pn + kstep : pn));
-    }
+    AxisK Kk;
+    if (V == 1 && ak) Kk.load(A, 3, k);   // (V = 4: 3% slower here than beside its use, V = 1: 8% faster)
+    filled();
     Vec<V> acc;
 #pragma unroll
     for (int j = 0; j < V; j++) acc.a[j] = 0.f;
@@ -420,6 +433,7 @@ __device__ __forceinline__ void march_cta(const MarchArgs& A, unsigned item) {
 #pragma unroll
       for (int j = 0; j < V; j++) acc.a[j] = div32(acc.a[j], f[j + 1], f[j], xh[j], xo[j]);
     }
+    commit();
     auto axis = [&](int a, int se, int sv, int sf, const unsigned o[4], const AxisK& K) {
       Vec<V> e[4];
 #pragma unroll
@@ -434,13 +448,21 @@ __device__ __forceinline__ void march_cta(const MarchArgs& A, unsigned item) {
       }
       both_faces<V>(acc, K, vr, vl, e[0], e[1], Ec, e[2], e[3]);
     };
+    filled();
     if (ay) axis(1, 1, 18, 23, oy, Ky);
+    commit();
+    filled();
     if (az) axis(2, 5, 19, 24, oz, Kz);
+    commit();
+    filled();
     if (ak) {
-      AxisK Kk;
-      Kk.load(A, 3, k);
+      if (V > 1) Kk.load(A, 3, k);
+      E2 = slot_take<V>(slot0);
       const Vec<V> vk = slot_take<V>(slot0 + 20 * SS);
-      if (more) slot_fill<V>(slot0 + 20 * SS, A.vel[3], pn);
+      if (more) {
+        slot_fill<V>(slot0, A.E, k + 3 < nk ? pn + 2u * kstep : (k + 2 < nk ? pn + kstep : pn));
+        slot_fill<V>(slot0 + 20 * SS, A.vel[3], pn);
+      }
       const Vec<V> D1 = vsub<V>(E2, E1);
       const Vec<V> fr = vflux<V>(vk, Kk.r, Dm, D0, D1, Ec, E1);
       vdiv<V>(acc, fr, fk, Kk.hi, Kk.lo);
@@ -448,11 +470,17 @@ __device__ __forceinline__ void march_cta(const MarchArgs& A, unsigned item) {
       Dm = D0;
       D0 = D1;
     }
+    commit();
+    filled();
     if (al) axis(4, 9, 21, 25, ol, Kl);
+    commit();
+    filled();
     if (am) axis(5, 13, 22, 26, om, Km);
+    commit();
+    filled();
     const Vec<V> lam = slot_take<V>(slot0 + 27 * SS);
     if (more) slot_fill<V>(slot0 + 27 * SS, A.lam, pn);
-    asm volatile("cp.async.commit_group;");
+    commit();
     // ---- mean-flow term and update ----
     Vec<V> out;
     if constexpr (V == 1) {
