@@ -198,7 +198,7 @@ int rt_get_tendency(rt_handle* h, double* dE, double* meanfl);
  *   15 = binary64: as 2
  *   16 = binary64 fast: without divisions (limiter slope selected exactly,
  *        update regrouped; its fields are allocated by this call: 58 bytes
- *        per cell and rings of slopes, 0.9 GB at 32^6 cells);
+ *        per cell and rings of slopes, 1.3 GB at 32^6 cells);
  *        within a few units in the last place of the reference's result per
  *        step, NOT bit-identical to it.  band and threads have no effect;
  *        fields of 2^31 cells or more are rejected (RT_ERR_CUDA on the step)

@@ -21,13 +21,16 @@
 //           values of a warp lie within 2^8 of each other (superbee_near64),
 //           one or two binary64 subtractions per face otherwise;
 //   role B  the update.
-// One launch gives half of its CTAs role A on one slab of the field and half
-// role B on the slab before, so that the integer and the binary64 pipes work
-// side by side: a launch at 20^6 has the binary64 pipe 56% busy, the issue
-// slots 63% and DRAM 62%.  Measured per step, against two launches of fluxes
-// (37 binary64 instructions per cell) and update: 32x32x32x12^3 4.30 -> 3.28
-// ms (3.56 with varying spacings), 32^6 81.3 -> 62.7 ms, 18x14x20x10x12x14
-// 677 -> 545 us (596).  (One launch for the whole step, its CTAs ordered by counters
+// One launch has CTAs of role A on one slab of the field and of role B on the
+// slab before in turns, so that the integer and the binary64 pipes work side
+// by side, and starts while the launch ahead drains.  32x32x32x12^3 has the
+// binary64 pipe 56% busy, the issue slots 60% and DRAM 67% (78% of the
+// measured copy rate: the slopes leave L2 before they are read), 58 warps per
+// SM; with 6, 5 and 4 CTAs per SM of more registers a step takes
+// 3.4, 3.8 and 3.8 ms.  Measured per step, against two launches of fluxes (37
+// binary64 instructions per cell) and update: 32x32x32x12^3 4.30 -> 3.15 ms
+// (3.48 with varying spacings), 32^6 81.3 -> 61.3 ms, 18x14x20x10x12x14 677 ->
+// 517 us (572).  (One launch for the whole step, its CTAs ordered by counters
 // of finished chunks, measured 5.8 ms against 3.2 at 32x32x32x12^3: CTAs wait
 // for one another and the slopes still go to memory.)
 //
@@ -192,15 +195,17 @@ __device__ __forceinline__ void fast_update(const Dims& d, const FastFields& C, 
     const int ca = c[a];
     const bool inl = signs >> a & 1u, inr = signs >> (6 + a) & 1u;
     const double Ein = E[inl || inr ? nb32(d, G, p, a, ca, inl ? -1 : +1, c[5]) : p];
-    const double Vr = C.V[a][p], Hr = C.H[a][p];
+    const double Vr = a < 4 ? C.V[a][p] : __ldcs(C.V[a] + p), Hr = a < 4 ? C.H[a][p] : __ldcs(C.H[a] + p);
     const double sr = C.psi[a][pu & C.mask[a]];
     // the left face: only addresses depend on where the cell is, so that no
-    // arithmetic stands in a branch (a warp would issue it for both sides)
+    // arithmetic stands in a branch (a warp would issue it for both sides).
+    // What nobody reads after this, or only a long way on (l, m), goes from
+    // L2 first: 3.20 -> 3.15 ms per step at 32x32x32x12^3.
     const bool in = ca > 0;
     const int q = in ? p - G.s[a] : plane32(G, a, c);
-    const double Vl = *((in ? C.V[a] : C.V0[a]) + q), Hl = *((in ? C.H[a] : C.H0[a]) + q);
+    const double Vl = __ldcs((in ? C.V[a] : C.V0[a]) + q), Hl = __ldcs((in ? C.H[a] : C.H0[a]) + q);
     const bool mirror = a == 2 && d.lower_refl;
-    const double ps = *((in || !mirror ? C.psi[a] : C.psi0) + ((in ? (unsigned)q : pu) & C.mask[a]));
+    const double ps = __ldcs((in || !mirror ? C.psi[a] : C.psi0) + ((in ? (unsigned)q : pu) & C.mask[a]));
     const double sl = in || mirror ? ps : 0.0;
     const double Vin = inflow(Vl, Vr, inl, inr);
     double t = UNI ? __fma_rn(Vin, Ein, acc) : __dmul_rn(Vin, Ein);
@@ -224,44 +229,58 @@ __device__ __forceinline__ void fast_update(const Dims& d, const FastFields& C, 
   if (valid) __stcs(Enew + p, __dadd_rn(e0, acc));
 }
 
-// slab A [a0, a1): slopes; slab B [b0, b1): update; with both, the CTAs take
-// turns
+// slab A [a0, a1): slopes, slab B [b0, b1): update; `lead` blocks of the one
+// role, then the two in turns, then what is left.  The launch may start
+// before the one ahead of it has ended: slopes depend on E alone, the update
+// waits until that launch is complete (and with it all before it, whose
+// completion its own update blocks waited for before they let this launch
+// start).  Rings hold the three slabs that are then in use.
 template <bool XW, bool UNI>
 __global__ void __launch_bounds__(256, 7)
     fast_step_kernel(const __grid_constant__ Dims d, const __grid_constant__ FastFields C,
                      const __grid_constant__ CellGeom G, const double* __restrict__ E, double* __restrict__ Enew,
-                     unsigned a0, unsigned a1, unsigned b0, unsigned b1) {
-  const bool two = a1 > a0 && b1 > b0;
-  const unsigned blk = two ? blockIdx.x >> 1 : blockIdx.x;
-  if (two ? !(blockIdx.x & 1) : a1 > a0) {
-    const unsigned first = a0 + blk * 256;
-    if (first < a1) fast_slopes<XW>(d, C, G, E, first + threadIdx.x, a1);
+                     unsigned a0, unsigned a1, unsigned b0, unsigned b1, unsigned lead, unsigned na, unsigned nb) {
+  bool slopes = true;
+  unsigned blk = blockIdx.x;
+  if (blk >= lead) {
+    const unsigned t = blk - lead;               // update, slopes, update, ... while both last
+    const unsigned turns = min(na - lead, nb);
+    slopes = t < 2 * turns ? (t & 1u) != 0 : na - lead > nb;
+    blk = t < 2 * turns ? t >> 1 : t - turns;
+    if (slopes) blk += lead;
+  }
+  if (slopes) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    fast_slopes<XW>(d, C, G, E, a0 + blk * 256 + threadIdx.x, a1);
   } else {
-    const unsigned first = b0 + blk * 256;
-    if (first < b1) fast_update<UNI>(d, C, G, E, Enew, first + threadIdx.x, b1);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+    fast_update<UNI>(d, C, G, E, Enew, b0 + blk * 256 + threadIdx.x, b1);
   }
 }
 
-// Cells of a slab: whole (x,y,z) volumes, at most 2^21 or from 2^25 cells on
-// 2^22 (less one volume, so that the rings of the short strides hold 2^22 and
-// 2^23 values), all slabs alike.  32x32x32x12^3 measured 3.62 ms per step at
-// 2^20, 3.35 at 2^21, 3.21 at 2^22 and 2^23 (the last wave of every launch);
-// 18x14x20x10x12x14 573, 539, 540 and 578 us (the first and last launch have
-// one role only).
+// Cells of a slab: whole (x,y,z) volumes, a quarter of the field within 2^19
+// and 2^22, all slabs alike.  At 2^19, 2^20, 2^21 and 2^22 cells
+// 32x32x32x12^3 (57 M) measured 3.43, 3.31, 3.24 and 3.20 ms per step,
+// 18x14x20x10x12x14 (8.5 M) 527, 516, 512 and 520 us (the first and the last
+// launch have one role only), 10x10x12x10x10x12 (1.4 M) 101, 103, 108, 108.
 long long slab_cells(const Dims& d) {
-  long long planes = (d.ncell >= (1ll << 25) ? 1ll << 22 : 1ll << 21) / d.nvol3 - 1;
-  if (planes < 1) planes = 1;
-  if (planes > d.nspec) planes = d.nspec;
+  const long long want = std::min(1ll << 22, std::max(1ll << 19, d.ncell / 4));
+  const long long planes = std::min((long long)d.nspec, std::max(1ll, want / d.nvol3));
   const long long slabs = (d.nspec + planes - 1) / planes;
   return (d.nspec + slabs - 1) / slabs * d.nvol3;
 }
+// blocks of slopes at the front of a launch: half of those the GPU holds, so
+// that the blocks which wait for the launch ahead do not fill it (0, 532 and
+// 1064 measured 3.40, 3.31 and 3.32 ms per step with slabs of 2^20 cells)
+constexpr unsigned kLead = 152 * 7 / 2;
 
 }  // namespace
 
-// ring of axis a: two slabs and the stride, a power of two
+// ring of axis a: three slabs and the stride, a power of two
 long long fast_ring(const Dims& d, int a) {
   if (d.n[a] <= 1) return 0;
-  const long long need = std::min(2 * slab_cells(d) + d.s[a], d.ncell);
+  const long long need = std::min(3 * slab_cells(d) + d.s[a], d.ncell);
   long long r = 1;
   while (r < need) r *= 2;
   return r;
@@ -290,10 +309,19 @@ cudaError_t launch_step_fast(const Dims& d, const FastFields& C, const double* E
   for (long long at = 0; at < d.ncell + slab; at += slab) {
     const long long a0 = std::min(at, d.ncell), a1 = std::min(at + slab, d.ncell);
     const long long b0 = std::max(0ll, at - slab), b1 = std::min(at, d.ncell);
-    const long long na = (a1 - a0 + 255) / 256, nb = (b1 - b0 + 255) / 256;
-    const long long blocks = na && nb ? 2 * std::max(na, nb) : na + nb;
-    kernel<<<(unsigned)blocks, 256, 0, st>>>(d, C, G, E, Enew, (unsigned)a0, (unsigned)a1, (unsigned)b0, (unsigned)b1);
-    const cudaError_t e = cudaGetLastError();
+    const unsigned na = (unsigned)((a1 - a0 + 255) / 256), nb = (unsigned)((b1 - b0 + 255) / 256);
+    const unsigned lead = nb ? std::min(na, kLead) : na;
+    cudaLaunchAttribute early;
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(na + nb);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cfg.attrs = &early;
+    cfg.numAttrs = at > 0 ? 1 : 0;   // the first launch reads what the step before wrote
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, d, C, G, E, Enew, (unsigned)a0, (unsigned)a1, (unsigned)b0,
+                                             (unsigned)b1, lead, na, nb);
     if (e != cudaSuccess) return e;
     *nlaunch += 1;
   }
