@@ -14,14 +14,14 @@
 // The bound is the binary64 pipe: 7 instructions per face flux (10 where
 // values next to each other differ by more than 2^8), two per axis in the
 // divergence and seven in the update, 61 per cell with six axes in the two
-// passes (290 with the divisions on that pipe).  32x32x32x12^3 measured 7.65
-// ms per step, 7.4 G cells/s and 451 G binary64 instructions/s, 85% of the
+// passes (290 with the divisions on that pipe).  32x32x32x12^3 measured 7.57
+// ms per step, 7.5 G cells/s and 456 G binary64 instructions/s, 86% of the
 // measured rate (9.45 ms with 10 per flux); the TMA plane kernel took 39.9
 // ms, and a CTA of 512 threads per x-y plane 280 us for a 40x120 column
-// (one launch here: 8.2 us), 6.3 ms for a 10x20x60x60 section (83 us) and
-// 8.7 ms for 8x8x16x16^3 (0.59 ms).  The integer work (340 instructions per
+// (one launch here: 8.2 us), 6.3 ms for a 10x20x60x60 section (79 us) and
+// 8.7 ms for 8x8x16x16^3 (0.58 ms).  The integer work (340 instructions per
 // flux) wants many warps to hide behind: 32 registers and 8 resident CTAs
-// with some spilling measured 7.65 ms, 40 and 6 CTAs 7.90, 48 and 5 CTAs
+// with some spilling measured 7.65 ms then, 40 and 6 CTAs 7.90, 48 and 5 CTAs
 // 8.15, 52 and 4 CTAs 8.40.
 #include <algorithm>
 
@@ -295,9 +295,18 @@ __device__ __forceinline__ double zero_minus(double q) {
   return __hiloint2double((int)(is_zero(b) ? 0u : b.hi ^ 0x80000000u), (int)b.lo);
 }
 
+// the launches of a step come one upon the other: a launch gets its blocks
+// ready while the one ahead drains, and each block waits until that one is
+// complete (a no-op where the launch was not told so)
+__device__ __forceinline__ void after_launch_ahead() {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // CACHED: uc holds the uCFL (it holds the fast step's h otherwise)
 template <bool CACHED>
 __global__ void __launch_bounds__(256, 8) exact_flux_kernel(StepArgs<double> A, SplitFluxes F, CellGeom G, Slab L) {
+  after_launch_ahead();
   const Dims& d = A.d;
   unsigned pu = L.base + blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = pu < L.end;
@@ -329,6 +338,7 @@ __global__ void __launch_bounds__(256, 8) exact_flux_kernel(StepArgs<double> A, 
 }
 
 __global__ void __launch_bounds__(256, 8) exact_update_kernel(StepArgs<double> A, SplitFluxes F, CellGeom G, Slab L) {
+  after_launch_ahead();
   const Dims& d = A.d;
   const unsigned pu = L.base + blockIdx.x * blockDim.x + threadIdx.x;
   if (pu >= L.end) return;
@@ -363,6 +373,15 @@ __global__ void __launch_bounds__(256, 8) exact_update_kernel(StepArgs<double> A
 // waves: a step of 8x8x16x16^3 measured 809 us at 2^19 cells, 739 at 2^20,
 // 703 at 2^22; 18x14x20x10x12x14 1587, 1587 and 1439 us.
 constexpr long long kSlabCells = 1ll << 21;
+// Blocks from which on the flux launch, too, gets ready beside the launch ahead:
+// chains of nothing but such launches come only every 16 us.  A step of
+// 10x20x60x60 (2813 blocks) measured 83.1 us with neither, 82.2 with the
+// update's and 78.9 with both, 16x32x30x32 (1920) 57.7, 57.3 and 53.8;
+// 10x20x30x40 (938) 36.9, 34.9 and 36.6, 10x20x24x24 (450) 20.5, 18.5 and
+// 32.7.  32x32x32x12^3: 7.65 and 7.57 ms.  (Fluxes and update of neighbouring
+// slabs side by side in one launch, as the fast step has them: 7.84 ms, and
+// three slabs of scratch.)
+constexpr unsigned kReadyBlocks = 1024;
 // Largest field stepped in one launch, both faces of every axis per cell
 // (twice the flux work, one launch less): 160x300 took 10.3 us against 14.4
 // in two passes, 6x6x8x6^3 (62,208 cells) 24.8 against 24.5, 10x20x24x24
@@ -492,11 +511,18 @@ cudaError_t launch_step_exact_slabs(const StepArgs<double>& A, const SplitFluxes
   for (int c0 = 0; c0 < d.n[ax]; c0 += m) {
     const Slab L = make_slab(d, ax, m, c0);
     const unsigned blocks = (L.end - L.base + 255) / 256;
-    exact_flux_kernel<true><<<blocks, 256, 0, st>>>(A, F, G, L);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    exact_update_kernel<<<blocks, 256, 0, st>>>(A, F, G, L);
-    e = cudaGetLastError();
+    cudaLaunchAttribute ready;
+    ready.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    ready.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cfg.attrs = &ready;
+    cfg.numAttrs = blocks >= kReadyBlocks ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, exact_flux_kernel<true>, A, F, G, L);
+    cfg.numAttrs = 1;
+    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, exact_update_kernel, A, F, G, L);
     if (e != cudaSuccess) return e;
     *nlaunch += 2;
   }
