@@ -8,16 +8,19 @@
 //   omega_kernel   evaluates the relation once per grid point into a scratch
 //                  ring of m planes (omega_e), with 1/omega_i of the interior
 //                  beside it;
-//   coeff_kernel   forms, per cell, the four pair sums of each axis pair,
+//   coeff_kernel   forms, walking along k, the pair sums of each axis pair,
 //                  both faces' velocities of all six axes from them (the left
 //                  faces of the first cells are the face-0 planes, all of
 //                  them enter the CFL rate), and the growth rates, and stores
 //                  them in the form's precision.
-// Divisions run on the integer pipes (rt_exact.cuh).  About 80 binary64
-// instructions and 27 integer quotients per cell; the values are those of the
+// Divisions, comparisons, changes of sign and the conversion to binary32 run
+// on the integer pipes (rt_exact.cuh).  About 62 binary64 instructions and 26
+// integer quotients per cell, both pipes near 70% busy; registers, not warps:
+// 2 to 4 CTAs per SM measure the same.  The values are those of the
 // reference's sequence bit for bit (rt_coeff.cuh states it).  24^3x12x12x16
-// (31.9 M cells) in binary32: 8.8 ms for all of it, against 60 ms for the
-// direct evaluation and its separate face-0, rate and conversion passes.
+// (31.9 M cells) in binary32: 7.0 ms for all of it (8.8 with a thread per cell and
+// those operations on the binary64 pipe), against 60 ms for the direct
+// evaluation and its separate face-0, rate and conversion passes.
 #include <algorithm>
 
 #include "rt_coeff.cuh"
@@ -84,11 +87,28 @@ __device__ __forceinline__ double half_slope(double A, double B, double dd) {
   return __ddiv_rn(dsub(dmul(0.5, A), dmul(0.5, B)), dd);
 }
 
-// outflow-only ends (calc_parameter.f90:55-66 etc.)
+// -x: written as such it becomes a binary64 instruction
+__device__ __forceinline__ double minus(double x) {
+  double r;
+  asm("{\n\t.reg .b64 t;\n\tmov.b64 t, %1;\n\txor.b64 t, t, 0x8000000000000000;\n\tmov.b64 %0, t;\n\t}" : "=d"(r) : "d"(x));
+  return r;
+}
+
+// outflow-only ends (calc_parameter.f90:55-66 etc.): max(0, v) and
+// -max(0, -v), compared as bit patterns (a NaN stays)
 __device__ __forceinline__ double clamp_face(double v, int f, int n, bool hi, bool lo) {
-  if (f == n && hi) v = fmax2(0.0, v);
-  if (f == 0 && lo) v = -fmax2(0.0, -v);
+  const uint64_t u = (uint64_t)__double_as_longlong(v);
+  const bool neg = u > 0x8000000000000000ull && u <= 0xfff0000000000000ull, pos = u - 1 < 0x7ff0000000000000ull;
+  if (f == n && hi && neg) v = 0.0;
+  if (f == 0 && lo && pos) v = __longlong_as_double((long long)0x8000000000000000ull);
   return v;
+}
+
+// fmax2 of two magnitudes (a > b ? a : b, NaN included)
+__device__ __forceinline__ double max_abs(double x, double y) {
+  const uint64_t a = (uint64_t)__double_as_longlong(x) & 0x7fffffffffffffffull;
+  const uint64_t b = (uint64_t)__double_as_longlong(y) & 0x7fffffffffffffffull;
+  return __longlong_as_double((long long)(a > b && a <= 0x7ff0000000000000ull ? a : b));
 }
 
 template <class T>
@@ -96,101 +116,137 @@ __device__ __forceinline__ T as(double x);
 template <>
 __device__ __forceinline__ double as<double>(double x) { return x; }
 template <>
-__device__ __forceinline__ float as<float>(double x) { return __double2float_rn(x); }
+__device__ __forceinline__ float as<float>(double x) { return float_rn(x); }
 
-// cells of the m planes [m0, m0 + gridDim.z) (Fortran m from 1); block (b,
-// u, j): spectral points u, u + gridDim.y, ... of plane m0 + j
+// cells of the m planes [m0, m0 + gridDim.z) (Fortran m from 1): a thread
+// takes a spatial cell at one (l,m) and walks klen values of k.  From one k to
+// the next it keeps what they share: omega at k + 1, the pair sums over the k
+// face between them and that face's spectral velocity; and what does not
+// depend on k (the shears of the growth rate, the indices) is formed once.
 template <class T>
 __global__ void __launch_bounds__(256, 2) coeff_kernel(Dims d, Background bg, Grid g, Phys ph, OmegaGeom G, int m0,
-                                                    const double* __restrict__ om, const double* __restrict__ inv,
-                                                    CoeffOut<T> out, unsigned long long* rate) {
+                                                       int segs, int klen, const double* __restrict__ om,
+                                                       const double* __restrict__ inv, CoeffOut<T> out,
+                                                       unsigned long long* rate) {
   unsigned long long best = 0;
-  for (unsigned u = blockIdx.y; u < (unsigned)(d.n[3] * d.n[4]); u += gridDim.y) {
-    int c[6];
-    c[3] = (int)(u % (unsigned)d.n[3]) + 1;
-    c[4] = (int)(u / (unsigned)d.n[3]) + 1;
-    c[5] = m0 + (int)blockIdx.z;
-    // offsets of the spectral points (l, n, m) and their neighbours
-    const long long o0 = (long long)(c[3] + G.wk * c[4]) * G.s3;
-    const double* w0 = om + (long long)(c[5] % G.ring) * G.plane + o0;
-    const double* wm[2] = {om + (long long)((c[5] - 1) % G.ring) * G.plane + o0,
-                           om + (long long)((c[5] + 1) % G.ring) * G.plane + o0};
-    const double* wl[2] = {w0 - (long long)G.wk * G.s3, w0 + (long long)G.wk * G.s3};
-    const double* wk[2] = {w0 - G.s3, w0 + G.s3};
-    const double ktv = g.kt[pidx(c[3])], ltv = g.lt[pidx(c[4])];
-    const long long sp = (long long)(c[3] - 1) + d.n[3] * ((c[4] - 1) + (long long)d.n[4] * (c[5] - 1));
+  const bool xk = d.n[0] > 1 && d.n[3] > 1;
+  int c[6];
+  c[5] = m0 + (int)blockIdx.z;
+  const double* plane = om + (long long)(c[5] % G.ring) * G.plane;
+  const double* below = om + (long long)((c[5] - 1) % G.ring) * G.plane;
+  const double* above = om + (long long)((c[5] + 1) % G.ring) * G.plane;
+  for (unsigned u = blockIdx.y; u < (unsigned)(d.n[4] * segs); u += gridDim.y) {
+    c[4] = (int)(u / (unsigned)segs) + 1;
+    const int k0 = (int)(u % (unsigned)segs) * klen + 1, k1 = min(k0 + klen - 1, d.n[3]);
+    const double ltv = g.lt[pidx(c[4])];
     for (unsigned v3 = blockIdx.x * blockDim.x + threadIdx.x; v3 < (unsigned)d.nvol3; v3 += gridDim.x * blockDim.x) {
       c[0] = (int)(v3 % (unsigned)d.n[0]) + 1;
       const unsigned r3 = v3 / (unsigned)d.n[0];
       c[1] = (int)(r3 % (unsigned)d.n[1]) + 1;
       c[2] = (int)(r3 / (unsigned)d.n[1]) + 1;
-      const long long p = v3 + sp * d.nvol3;
       const int w = c[0] + G.sx * (c[1] + G.sy * c[2]);
       const int back[3] = {1, G.sx, G.sx * G.sy};
       const long long q = bg_idx(bg, c[0], c[1], c[2]);
-      const double e0 = w0[w];
-      double vr[6], vl[6];
-  #pragma unroll
-      for (int s = 0; s < 3; s++) {
-        const int a = s, b = s + 3;
-        if (s < 2 && !(d.n[a] > 1 && d.n[b] > 1)) {
-          // collapsed x/k or y/l pair: analytic spatial velocity on interior cells
-          const int cl[6] = {c[0] - (s == 0), c[1] - (s == 1), c[2], c[3], c[4], c[5]};
-          vr[a] = analytic_vel(bg, g, ph, c, s);
-          vl[a] = cl[a] >= 1 ? analytic_vel(bg, g, ph, cl, s) : 0.0;
-          vr[b] = vl[b] = 0.0;
-          continue;
-        }
-        const double* lo = s == 0 ? wk[0] : (s == 1 ? wl[0] : wm[0]);
-        const double* hi = s == 0 ? wk[1] : (s == 1 ? wl[1] : wm[1]);
-        const int wb = w - back[s];
-        const double eb = w0[wb];
-        // pair sums of aloc (twice the average over the wavenumber neighbours)
-        const double A00 = dadd(e0, hi[w]), A01 = dadd(lo[w], e0);     // at (cell, w), (cell, w - 1)
-        const double A10 = dadd(eb, hi[wb]), A11 = dadd(lo[wb], eb);   // at the spatial neighbour below
-        const double ds = g.d[a][pidx(c[a])], dw = g.d[b][pidx(c[b])];
-        const bool up = s < 2 || !d.upper_refl, dn = s < 2 || !d.lower_refl;
-        vr[a] = clamp_face(half_slope(A00, A01, dw), c[a], d.n[a], up, dn);
-        vl[a] = clamp_face(half_slope(A10, A11, dw), c[a] - 1, d.n[a], up, dn);
-        vr[b] = clamp_face(-half_slope(A00, A10, ds), c[b], d.n[b], true, true);
-        vl[b] = clamp_face(-half_slope(A01, A11, ds), c[b] - 1, d.n[b], true, true);
-      }
-      double r = 0.0;
-  #pragma unroll
-      for (int a = 0; a < 6; a++) {
-        out.vel[a][p] = as<T>(vr[a]);
-        if (c[a] == 1) {
-          long long f = 0;
-  #pragma unroll
-          for (int b = 0; b < 6; b++) f += (long long)(c[b] - 1) * d.ps[a][b];
-          out.vlo[a][f] = as<T>(vl[a]);
-        }
-        if (d.n[a] > 1) r = dadd(r, div_rn(fmax2(fabs(vl[a]), fabs(vr[a])), g.d[a][pidx(c[a])]));
-      }
-      const unsigned long long rb = (unsigned long long)__double_as_longlong(r) & 0x7fffffffffffffffull;
-      best = rb > best ? rb : best;
-      // growth rates, calc_parameter.f90:246-254
-      const double iv = inv[(long long)(c[5] % G.ring) * d.s[5] + (p - (long long)(c[5] - 1) * d.s[5])];
-      const double xu = dsub(vr[0], bg.U[q]), yv = dsub(vr[1], bg.V[q]);
       const long long st[3] = {1, bg.px, (long long)bg.px * bg.py};
-      double lam[3];
+      double dU[3], dV[3];
   #pragma unroll
       for (int s = 0; s < 3; s++) {
-        const double d2 = dmul(2.0, g.d[s][pidx(c[s])]);
-        const double dU = dsub(bg.U[q + st[s]], bg.U[q - st[s]]), dV = dsub(bg.V[q + st[s]], bg.V[q - st[s]]);
-        const double f1 = s < 2 ? xu : ktv, f2 = s < 2 ? yv : ltv;
-        const double head = dmul(iv, s == 0 ? ktv : (s == 1 ? ltv : vr[2]));
-        lam[s] = dmul(head, dadd(div_rn(dmul(f1, dU), d2), div_rn(dmul(f2, dV), d2)));
+        dU[s] = dsub(bg.U[q + st[s]], bg.U[q - st[s]]);
+        dV[s] = dsub(bg.V[q + st[s]], bg.V[q - st[s]]);
       }
-      if constexpr (sizeof(T) == 8) {
+      long long o = (long long)(k0 + G.wk * c[4]) * G.s3;   // (k, l) of the walk in an omega plane
+      double e0 = plane[o + w], ebx = 0.0, A01x = 0.0, A11x = 0.0, hk = 0.0;
+      if (xk) {
+        ebx = plane[o + w - 1];
+        A01x = dadd(plane[o - G.s3 + w], e0);
+        A11x = dadd(plane[o - G.s3 + w - 1], ebx);
+        hk = half_slope(A01x, A11x, g.d[0][pidx(c[0])]);
+      }
+      for (c[3] = k0; c[3] <= k1; c[3]++, o += G.s3) {
+        const double ktv = g.kt[pidx(c[3])];
+        const long long p = v3 + d.nvol3 * ((long long)(c[3] - 1) + d.n[3] * ((c[4] - 1) + (long long)d.n[4] * (c[5] - 1)));
+        double vr[6], vl[6], e1 = 0.0;
+        if (xk) {
+          e1 = plane[o + G.s3 + w];
+          const double eb1 = plane[o + G.s3 + w - 1];
+          // pair sums of aloc (twice the average over the wavenumber neighbours)
+          const double A00 = dadd(e0, e1), A10 = dadd(ebx, eb1);   // at (cell, k), (the cell below, k)
+          const double dw = g.d[3][pidx(c[3])], hr = half_slope(A00, A10, g.d[0][pidx(c[0])]);
+          vr[0] = clamp_face(half_slope(A00, A01x, dw), c[0], d.n[0], true, true);
+          vl[0] = clamp_face(half_slope(A10, A11x, dw), c[0] - 1, d.n[0], true, true);
+          vr[3] = clamp_face(minus(hr), c[3], d.n[3], true, true);
+          vl[3] = clamp_face(minus(hk), c[3] - 1, d.n[3], true, true);
+          A01x = A00;
+          A11x = A10;
+          ebx = eb1;
+          hk = hr;
+        }
   #pragma unroll
-        for (int s = 0; s < 3; s++) out.lam[s][p] = lam[s];
-      } else {   // one combined rate, summed in binary64 before rounding
-        double sum = 0.0;
+        for (int s = 0; s < 3; s++) {
+          const int a = s, b = s + 3;
+          if (s < 2 && !(d.n[a] > 1 && d.n[b] > 1)) {
+            // collapsed x/k or y/l pair: analytic spatial velocity on interior cells
+            const int cl[6] = {c[0] - (s == 0), c[1] - (s == 1), c[2], c[3], c[4], c[5]};
+            vr[a] = analytic_vel(bg, g, ph, c, s);
+            vl[a] = cl[a] >= 1 ? analytic_vel(bg, g, ph, cl, s) : 0.0;
+            vr[b] = vl[b] = 0.0;
+            continue;
+          }
+          if (s == 0) continue;
+          const double* lo = s == 1 ? plane + o - (long long)G.wk * G.s3 : below + o;
+          const double* hi = s == 1 ? plane + o + (long long)G.wk * G.s3 : above + o;
+          const int wb = w - back[s];
+          const double eb = plane[o + wb];
+          const double A00 = dadd(e0, hi[w]), A01 = dadd(lo[w], e0);     // at (cell, w), (cell, w - 1)
+          const double A10 = dadd(eb, hi[wb]), A11 = dadd(lo[wb], eb);   // at the spatial neighbour below
+          const double ds = g.d[a][pidx(c[a])], dw = g.d[b][pidx(c[b])];
+          const bool up = s < 2 || !d.upper_refl, dn = s < 2 || !d.lower_refl;
+          vr[a] = clamp_face(half_slope(A00, A01, dw), c[a], d.n[a], up, dn);
+          vl[a] = clamp_face(half_slope(A10, A11, dw), c[a] - 1, d.n[a], up, dn);
+          vr[b] = clamp_face(minus(half_slope(A00, A10, ds)), c[b], d.n[b], true, true);
+          vl[b] = clamp_face(minus(half_slope(A01, A11, ds)), c[b] - 1, d.n[b], true, true);
+        }
+        e0 = xk ? e1 : (c[3] < k1 ? plane[o + G.s3 + w] : 0.0);
+        double r = 0.0;
+        bool first = true;   // (0 + x = x: no binary64 instruction for the first)
   #pragma unroll
-        for (int s = 0; s < 3; s++)
-          if (d.n[s] > 1) sum += lam[s];
-        out.lam[0][p] = as<T>(sum);
+        for (int a = 0; a < 6; a++) {
+          out.vel[a][p] = as<T>(vr[a]);
+          if (c[a] == 1) {
+            long long f = 0;
+  #pragma unroll
+            for (int b = 0; b < 6; b++) f += (long long)(c[b] - 1) * d.ps[a][b];
+            out.vlo[a][f] = as<T>(vl[a]);
+          }
+          if (d.n[a] > 1) {
+            const double t = div_rn(max_abs(vl[a], vr[a]), g.d[a][pidx(c[a])]);
+            r = first ? t : dadd(r, t);
+            first = false;
+          }
+        }
+        const unsigned long long rb = (unsigned long long)__double_as_longlong(r) & 0x7fffffffffffffffull;
+        best = rb > best ? rb : best;
+        // growth rates, calc_parameter.f90:246-254
+        const double iv = inv[(long long)(c[5] % G.ring) * d.s[5] + (p - (long long)(c[5] - 1) * d.s[5])];
+        const double xu = dsub(vr[0], bg.U[q]), yv = dsub(vr[1], bg.V[q]);
+        double lam[3];
+  #pragma unroll
+        for (int s = 0; s < 3; s++) {
+          const double d2 = dmul(2.0, g.d[s][pidx(c[s])]);
+          const double f1 = s < 2 ? xu : ktv, f2 = s < 2 ? yv : ltv;
+          const double head = dmul(iv, s == 0 ? ktv : (s == 1 ? ltv : vr[2]));
+          lam[s] = dmul(head, dadd(div_rn(dmul(f1, dU[s]), d2), div_rn(dmul(f2, dV[s]), d2)));
+        }
+        if constexpr (sizeof(T) == 8) {
+  #pragma unroll
+          for (int s = 0; s < 3; s++) out.lam[s][p] = lam[s];
+        } else {   // one combined rate, summed in binary64 before rounding
+          double sum = 0.0;
+  #pragma unroll
+          for (int s = 0; s < 3; s++)
+            if (d.n[s] > 1) sum += lam[s];
+          out.lam[0][p] = as<T>(sum);
+        }
       }
     }
   }
@@ -217,6 +273,8 @@ OmegaGeom make_omega(const Dims& d, int ring) {
   return G;
 }
 
+constexpr long long kBusy = 152 * 2 * 6;   // blocks
+
 unsigned walk_blocks(long long points) { return (unsigned)std::min<long long>((points + 255) / 256, 16); }
 
 }  // namespace
@@ -239,15 +297,21 @@ cudaError_t launch_coeff(const Dims& d, const Background& bg, const Grid& g, con
   if (e != cudaSuccess) return e;
   *nlaunch = 0;
   const int batch = ring - 2;
-  const unsigned wspec = (unsigned)std::min(G.wk * G.wl, 65535), spec = (unsigned)std::min(d.n[3] * d.n[4], 65535);
+  const unsigned wspec = (unsigned)std::min(G.wk * G.wl, 65535);
   for (int m0 = 1; m0 <= d.n[5]; m0 += batch) {
     const int cnt = std::min(batch, d.n[5] - m0 + 1);
     // planes 0 and 1 come with the first batch; then one beyond the last cell plane
     const int w0 = m0 == 1 ? 0 : m0 + 1, wn = m0 + cnt + 1 - w0;
     omega_kernel<<<dim3(walk_blocks(G.s3), wspec, (unsigned)wn), 256, 0, st>>>(d, bg, g, ph, G, w0, om, inv);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    coeff_kernel<T><<<dim3(walk_blocks(d.nvol3), spec, (unsigned)cnt), 256, 0, st>>>(
-        d, bg, g, ph, G, m0, om, inv, out, reinterpret_cast<unsigned long long*>(rate));
+    // walks along k as long as the GPU stays busy for a few rounds
+    const long long blocks = (d.nvol3 + 255) / 256 * d.n[4] * cnt;
+    const int want = (int)std::max(1ll, std::min<long long>(d.n[3], (kBusy + blocks - 1) / blocks));
+    const int klen = (d.n[3] + want - 1) / want, segs = (d.n[3] + klen - 1) / klen;
+    const dim3 grid((unsigned)((d.nvol3 + 255) / 256), (unsigned)std::min<long long>((long long)d.n[4] * segs, 65535),
+                    (unsigned)cnt);
+    coeff_kernel<T><<<grid, 256, 0, st>>>(d, bg, g, ph, G, m0, segs, klen, om, inv, out,
+                                          reinterpret_cast<unsigned long long*>(rate));
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     *nlaunch += 2;
   }

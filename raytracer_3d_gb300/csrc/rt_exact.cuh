@@ -147,6 +147,26 @@ __host__ __device__ __forceinline__ double div_rn(double a, double b) {
   return r;
 }
 
+// x to binary32, to nearest even, without the conversion instruction (which
+// shares the binary64 pipe) where the result is a normal number or zero
+__host__ __device__ __forceinline__ float float_rn(double x) {
+  const Bits64 b = split64(x);
+  const bool zero = is_zero(b);
+  const uint32_t low = b.lo & 0x1fffffffu;
+  uint32_t r = (uint32_t)((((uint64_t)(b.hi & 0x7fffffffu) << 32) | b.lo) >> 29) - (896u << 23);
+  r += low + (r & 1u) > 0x10000000u ? 1u : 0u;
+  r = (zero ? 0u : r) | (b.hi & 0x80000000u);
+  float f;
+#ifdef __CUDA_ARCH__
+  f = __uint_as_float(r);
+  if ((unsigned)(expo(b) - 897) >= 253u && !zero) f = __double2float_rn(x);
+#else
+  std::memcpy(&f, &r, 4);
+  if ((unsigned)(expo(b) - 897) >= 253u && !zero) f = (float)x;
+#endif
+  return f;
+}
+
 // Limiter(up/Rj) for Rj != 0 of superbee_fluxes.f90:10, :21-25:
 // max(0, min(1, 2r), min(2, r)) with r = up/Rj correctly rounded.  r <= 0
 // gives 0; r >= 2 gives 2 (also where only the rounded r reaches it); in

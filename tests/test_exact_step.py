@@ -106,6 +106,18 @@ def test_integer_differences_on_the_gpu(tmp_path):
     _check(tmp_path, src=os.path.join(ROOT, "tests", "native", "flux_near_check.cu"))
 
 
+FLOAT = os.path.join(ROOT, "tests", "native", "float_rn_check.cu")
+
+
+def test_conversion_to_binary32_on_the_host(tmp_path):
+    _check(tmp_path, src=FLOAT)
+
+
+@pytest.mark.gpu
+def test_conversion_to_binary32_on_the_gpu(tmp_path):
+    _check(tmp_path, "--device", src=FLOAT)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("scale", [1.0, 2.0 ** -262])   # the second: next to the end of the integer range
 @pytest.mark.parametrize("n", [(16, 16, 64, 2, 70, 1), (15, 7, 12, 10, 12, 16)])
