@@ -96,8 +96,12 @@ cudaError_t go(K kernel, int V, unsigned ctas, const P& args, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// CTAs that keep the GPU busy for a few rounds
-constexpr long long kBusy = 152 * 3 * 4;
+// CTAs a field should have: two rounds of what the GPU holds.  More segments
+// cost more starts than their even end saves: four rounds measured 76.6 us
+// per step at 16^3x12^3 against 73.8, 30.8 against 26.9 at 16^3x8^3, 20.5
+// against 16.4 at 8^3x12^3; one round 28.8 and 16.4 us.  From 20 M cells on
+// walks are whole either way.
+constexpr long long kBusy = 152 * 3 * 2;
 
 }  // namespace
 
