@@ -299,8 +299,8 @@ __device__ __forceinline__ double zero_minus(double q) {
 // ready while the one ahead drains, and each block waits until that one is
 // complete (a no-op where the launch was not told so)
 __device__ __forceinline__ void after_launch_ahead() {
-  asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
 }
 
 // CACHED: uc holds the uCFL (it holds the fast step's h otherwise)
@@ -373,12 +373,12 @@ __global__ void __launch_bounds__(256, 8) exact_update_kernel(StepArgs<double> A
 // waves: a step of 8x8x16x16^3 measured 809 us at 2^19 cells, 739 at 2^20,
 // 703 at 2^22; 18x14x20x10x12x14 1587, 1587 and 1439 us.
 constexpr long long kSlabCells = 1ll << 21;
-// Blocks from which on the flux launch, too, gets ready beside the launch ahead:
-// chains of nothing but such launches come only every 16 us.  A step of
-// 10x20x60x60 (2813 blocks) measured 83.1 us with neither, 82.2 with the
-// update's and 78.9 with both, 16x32x30x32 (1920) 57.7, 57.3 and 53.8;
-// 10x20x30x40 (938) 36.9, 34.9 and 36.6, 10x20x24x24 (450) 20.5, 18.5 and
-// 32.7.  32x32x32x12^3: 7.65 and 7.57 ms.  (Fluxes and update of neighbouring
+// Blocks from which on the flux launch, too, gets ready beside the launch ahead.
+// A step of 10x20x60x60 (2813 blocks) measured 83.1 us with neither, 82.2
+// with the update's and 78.9 with both, 16x32x30x32 (1920) 57.7, 57.3 and
+// 53.8; of smaller ones some lose: 10x20x30x40 (938) 36.9, 34.8 and 36.4,
+// 5x6x7x12x10x8 (788) 43.7, 41.2 and 49.5, 10x20x24x24 (450) 20.5, 18.5 and
+// 16.7.  32x32x32x12^3: 7.65 and 7.57 ms.  (Fluxes and update of neighbouring
 // slabs side by side in one launch, as the fast step has them: 7.84 ms, and
 // three slabs of scratch.)
 constexpr unsigned kReadyBlocks = 1024;
