@@ -4,7 +4,7 @@ Workload (N=1): the 32^3 x 32^3 wave field with a mean flow
 U = 0.1 sin(2 pi y/Ly) exp(z/500), log-normal spectrum, CFL 0.4, plain
 binary64 form (1,073,741,824 cells per step).  A step is one forward-Euler
 time step of the whole field with the schedule the autotuner picks (the
-division-free two-pass step: flux pass and update pass, two launches).
+division-free step, slopes and update of its slabs side by side).
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
 
@@ -273,7 +273,7 @@ def fp64_peak():
 
 
 # committed per-cell DRAM traffic (profiles/dram_traffic.json) of each timed binary32 kernel
-FP32_TRAFFIC = {"w2z": "step_fp32_w2z", "w2q": "step_fp32_w2q", "w3": "step_fp32_w3"}
+FP32_TRAFFIC = {"w2z": "step_fp32_w2z", "w2q": "step_fp32_march", "tma": "step_fp32_march", "w3": "step_fp32_w3"}
 
 SCHEDULE_NOTES = {
     "fast": "without divisions, slopes on the integer pipes (rt_fast.cu): within 1e-12 relative L-inf of the reference per step, "
@@ -604,7 +604,7 @@ def gpu_arm(args):
         main = run_form("fp64", n, args.steps, args.warmup, dist, args.e2e_steps, FP64_CANDIDATES[-1],
                         tune=args.tune, candidates=FP64_CANDIDATES, final_step=err_steps)
     f64_sched = tuple(main["schedule"])
-    f64_key = {"split": "step_fp64_split", "fast": "step_fp64_fast"}.get(f64_sched[0], "step_fp64")
+    f64_key = {"fast": "step_fp64_fast"}.get(f64_sched[0], "step_fp64_split")
     forms = {}
     if not args.no_fp32:
         f32 = run_form("fp32", n, args.steps, args.warmup, dist, 0, sched, tune=args.tune, final_step=err_steps)
