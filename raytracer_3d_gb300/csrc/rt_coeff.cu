@@ -13,14 +13,15 @@
 //                  faces of the first cells are the face-0 planes, all of
 //                  them enter the CFL rate), and the growth rates, and stores
 //                  them in the form's precision.
-// Divisions, comparisons, changes of sign and the conversion to binary32 run
-// on the integer pipes (rt_exact.cuh).  About 62 binary64 instructions and 26
-// integer quotients per cell, both pipes near 70% busy; registers, not warps:
+// Divisions, square roots, comparisons, changes of sign and the conversion to
+// binary32 run on the integer pipes (rt_exact.cuh).  About 62 binary64
+// instructions and 26 integer quotients per cell, both pipes near 70% busy; registers, not warps:
 // 2 to 4 CTAs per SM measure the same.  The values are those of the
 // reference's sequence bit for bit (rt_coeff.cuh states it).  24^3x12x12x16
-// (31.9 M cells) in binary32: 7.0 ms for all of it (8.8 with a thread per cell and
-// those operations on the binary64 pipe), against 60 ms for the direct
-// evaluation and its separate face-0, rate and conversion passes.
+// (31.9 M cells) in binary32: 6.2 ms for all of it (omega_kernel 1.0, 1.75
+// with the square root on the binary64 pipe; 8.8 with a thread per cell and
+// those operations there), against 60 ms for the direct evaluation and its
+// separate face-0, rate and conversion passes.
 #include <algorithm>
 
 #include "rt_coeff.cuh"
@@ -65,7 +66,7 @@ __global__ void __launch_bounds__(256) omega_kernel(Dims d, Background bg, Grid 
       const unsigned r = v / (unsigned)G.sx;
       const int j = (int)(r % (unsigned)G.sy), k = (int)(r / (unsigned)G.sy);
       const long long q = bg_idx(bg, i, j, k);
-      const double oi = sign_times(ph.sgn, __dsqrt_rn(div_rn(dadd(dmul(bg.Nsqr[q], kh2), f2m2), den)));
+      const double oi = sign_times(ph.sgn, sqrt_rn(div_rn(dadd(dmul(bg.Nsqr[q], kh2), f2m2), den)));
       out[v] = dadd(dadd(oi, dmul(ktv, bg.U[q])), dmul(ltv, bg.V[q]));
       if (inside && i > 0 && j > 0 && k > 0)
         outi[(i - 1) + d.n[0] * ((j - 1) + (long long)d.n[1] * (k - 1))] = div_rn(1.0, oi);

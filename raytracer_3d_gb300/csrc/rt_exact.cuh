@@ -147,6 +147,54 @@ __host__ __device__ __forceinline__ double div_rn(double a, double b) {
   return r;
 }
 
+// sqrt(x), correctly rounded, on the integer pipes: two digits of the root of
+// the significand from an approximate reciprocal root, the remainder kept
+// exactly (the longhand method with large digits).  The root of a binary64
+// number is never half-way between two of them, so the 54th bit alone decides
+// the rounding.
+__host__ __device__ __forceinline__ double sqrt_rn(double x) {
+  const Bits64 b = split64(x);
+  if (!((int)b.hi >= 0 && (unsigned)(expo(b) - 1) < 2046u)) {   // zero, denormal, negative, infinite, NaN
+#ifdef __CUDA_ARCH__
+    return __dsqrt_rn(x);
+#else
+    return __builtin_sqrt(x);
+#endif
+  }
+  const int E = expo(b) - 1023;
+  const uint64_t m = significand(b) << (E & 1);               // x = m/2^52 * 4^(E >> 1), m/2^52 in [1, 4)
+  // reciprocal root of the first 24 bits, lowered by eight units in the last
+  // place (the instruction is within two): below the true one by less than 2^-19.8
+  const uint32_t fb = (127u << 23) + ((E & 1) ? (1u << 23) : 0u) + ((b.hi & 0xfffffu) << 3) + (b.lo >> 29);
+  float f, r;
+#ifdef __CUDA_ARCH__
+  f = __uint_as_float(fb);
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(f));
+  const uint32_t rb = __float_as_uint(r) - 8u;
+#else
+  std::memcpy(&f, &fb, 4);
+  r = 1.0f / __builtin_sqrtf(f);
+  uint32_t rb;
+  std::memcpy(&rb, &r, 4);
+  rb = rb - 8u + RT_RECIP_HOST_ULP;
+#endif
+  const uint32_t g = (rb & 0x7fffffu) | 0x800000u;
+  uint32_t Y = (rb >> 23) >= 126u ? g << 8 : g << 7;          // y*2^32
+  const uint32_t a = (uint32_t)(m >> 22);                     // m/2^52 * 2^30, truncated
+  const uint32_t e = 0x3ffffffeu - mulhi32(mulhi32(Y, Y), a); // 2^30*(1 - a*y^2) or up to two less, > 0
+  Y += mulhi32(Y, e << 1);
+  const uint32_t s1 = mulhi32(a, Y);                          // root*2^30 or up to six less
+  const uint64_t R1 = (m << 8) - (uint64_t)s1 * s1;           // < 2^35
+  uint64_t T = ((uint64_t)s1 << 23) + (mulhi32((uint32_t)(R1 >> 3), Y) >> 5);   // floor(root*2^53) or up to two less
+  uint64_t R2 = (m << 54) - T * T;                            // exact modulo 2^64
+  if (R2 > 2 * T) {
+    R2 -= 2 * T + 1;
+    T++;
+  }
+  if (R2 > 2 * T) T++;
+  return join64(((uint64_t)(uint32_t)(1022 + (E >> 1)) << 52) + ((T + 1) >> 1));
+}
+
 // x to binary32, to nearest even, without the conversion instruction (which
 // shares the binary64 pipe) where the result is a normal number or zero
 __host__ __device__ __forceinline__ float float_rn(double x) {

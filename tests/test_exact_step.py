@@ -118,6 +118,19 @@ def test_conversion_to_binary32_on_the_gpu(tmp_path):
     _check(tmp_path, "--device", src=FLOAT)
 
 
+SQRT = os.path.join(ROOT, "tests", "native", "sqrt_rn_check.cu")
+
+
+@pytest.mark.parametrize("ulp", ["0", "2u", "0xfffffffeu"])
+def test_square_root_on_the_host(tmp_path, ulp):
+    _check(tmp_path, src=SQRT, flags=("-DRT_RECIP_HOST_ULP=" + ulp,))
+
+
+@pytest.mark.gpu
+def test_square_root_on_the_gpu(tmp_path):
+    _check(tmp_path, "--device", src=SQRT)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("scale", [1.0, 2.0 ** -262])   # the second: next to the end of the integer range
 @pytest.mark.parametrize("n", [(16, 16, 64, 2, 70, 1), (15, 7, 12, 10, 12, 16)])
