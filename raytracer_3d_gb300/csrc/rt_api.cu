@@ -1284,7 +1284,7 @@ int rt_calc_parameter(rt_handle* h) {
   // (taking 1.4 MB from the stream-ordered pool and giving it back cost 0.3 ms)
   double* scratch = nullptr;
   int ring = coeff_ring(d, 256ll << 20);
-  const bool small = coeff_scratch(d, ring) * (long long)sizeof(double) <= (4ll << 20);
+  const bool small = coeff_scratch(d, ring) * (long long)sizeof(double) <= (16ll << 20);
   int rc = RT_OK;
   if (small) {
     if (!h->coeff_mem) rc = dev_alloc(h, (void**)&h->coeff_mem, (size_t)coeff_scratch(d, ring) * sizeof(double));

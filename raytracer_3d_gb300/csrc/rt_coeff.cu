@@ -32,10 +32,12 @@ namespace rt {
 
 namespace {
 
-// points of the scratch: spatial indices 0..n, spectral indices 0..n+1 (Fortran)
+// points of the scratch: spatial indices 0..n, spectral indices 0..n+1
+// (Fortran); of an x/k or y/l pair whose velocities are analytic 1..n of both
 struct OmegaGeom {
-  int sx, sy, sz;        // spatial points per axis (n + 1)
-  int wk, wl;            // spectral points along k and l (n + 2)
+  int sx, sy, sz;        // spatial points per axis
+  int wk, wl;            // spectral points along k and l
+  int lo[2];             // first index of the x/k and y/l pairs
   unsigned s3;           // sx*sy*sz
   long long plane;       // doubles of one m plane: s3*wk*wl
   int ring;              // planes of the ring; plane m at m % ring
@@ -54,7 +56,7 @@ __global__ void __launch_bounds__(256) omega_kernel(Dims d, Background bg, Grid 
   const double m2 = dmul(mtv, mtv);
   const double f2m2 = dmul(dmul(ph.f0, ph.f0), m2);
   for (unsigned u = blockIdx.y; u < (unsigned)(G.wk * G.wl); u += gridDim.y) {
-    const int l = (int)(u % (unsigned)G.wk), n = (int)(u / (unsigned)G.wk);
+    const int l = G.lo[0] + (int)(u % (unsigned)G.wk), n = G.lo[1] + (int)(u / (unsigned)G.wk);
     const double ktv = g.kt[pidx(l)], ltv = g.lt[pidx(n)];
     const double kh2 = dadd(dmul(ltv, ltv), dmul(ktv, ktv));
     const double den = dadd(m2, kh2);
@@ -62,9 +64,9 @@ __global__ void __launch_bounds__(256) omega_kernel(Dims d, Background bg, Grid 
     const bool inside = l >= 1 && l <= d.n[3] && n >= 1 && n <= d.n[4] && m >= 1 && m <= d.n[5];
     double* outi = inv + (long long)(m % G.ring) * d.s[5] + (long long)((l - 1) + d.n[3] * (n - 1)) * d.nvol3;
     for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < G.s3; v += gridDim.x * blockDim.x) {
-      const int i = (int)(v % (unsigned)G.sx);
+      const int i = G.lo[0] + (int)(v % (unsigned)G.sx);
       const unsigned r = v / (unsigned)G.sx;
-      const int j = (int)(r % (unsigned)G.sy), k = (int)(r / (unsigned)G.sy);
+      const int j = G.lo[1] + (int)(r % (unsigned)G.sy), k = (int)(r / (unsigned)G.sy);
       const long long q = bg_idx(bg, i, j, k);
       const double oi = sign_times(ph.sgn, sqrt_rn(div_rn(dadd(dmul(bg.Nsqr[q], kh2), f2m2), den)));
       out[v] = dadd(dadd(oi, dmul(ktv, bg.U[q])), dmul(ltv, bg.V[q]));
@@ -145,7 +147,7 @@ __global__ void __launch_bounds__(256, 2) coeff_kernel(Dims d, Background bg, Gr
       const unsigned r3 = v3 / (unsigned)d.n[0];
       c[1] = (int)(r3 % (unsigned)d.n[1]) + 1;
       c[2] = (int)(r3 / (unsigned)d.n[1]) + 1;
-      const int w = c[0] + G.sx * (c[1] + G.sy * c[2]);
+      const int w = c[0] - G.lo[0] + G.sx * (c[1] - G.lo[1] + G.sy * c[2]);
       const int back[3] = {1, G.sx, G.sx * G.sy};
       const long long q = bg_idx(bg, c[0], c[1], c[2]);
       const long long st[3] = {1, bg.px, (long long)bg.px * bg.py};
@@ -155,7 +157,7 @@ __global__ void __launch_bounds__(256, 2) coeff_kernel(Dims d, Background bg, Gr
         dU[s] = dsub(bg.U[q + st[s]], bg.U[q - st[s]]);
         dV[s] = dsub(bg.V[q + st[s]], bg.V[q - st[s]]);
       }
-      long long o = (long long)(k0 + G.wk * c[4]) * G.s3;   // (k, l) of the walk in an omega plane
+      long long o = (long long)(k0 - G.lo[0] + G.wk * (c[4] - G.lo[1])) * G.s3;   // (k, l) of the walk in an omega plane
       double e0 = plane[o + w], ebx = 0.0, A01x = 0.0, A11x = 0.0, hk = 0.0;
       if (xk) {
         ebx = plane[o + w - 1];
@@ -263,11 +265,14 @@ __global__ void __launch_bounds__(256, 2) coeff_kernel(Dims d, Background bg, Gr
 
 OmegaGeom make_omega(const Dims& d, int ring) {
   OmegaGeom G;
-  G.sx = d.n[0] + 1;
-  G.sy = d.n[1] + 1;
+  const int xk = d.n[0] > 1 && d.n[3] > 1, yl = d.n[1] > 1 && d.n[4] > 1;
+  G.lo[0] = 1 - xk;
+  G.lo[1] = 1 - yl;
+  G.sx = d.n[0] + xk;
+  G.sy = d.n[1] + yl;
   G.sz = d.n[2] + 1;
-  G.wk = d.n[3] + 2;
-  G.wl = d.n[4] + 2;
+  G.wk = d.n[3] + 2 * xk;
+  G.wl = d.n[4] + 2 * yl;
   G.s3 = (unsigned)G.sx * G.sy * G.sz;
   G.plane = (long long)G.s3 * G.wk * G.wl;
   G.ring = ring;
