@@ -49,7 +49,7 @@ struct rt_handle {
   int cur = 0;
   int forcing = RT_FORCING_NONE;  // set_forcing before every step (rt_set_forcing)
   double* force = nullptr;      // its interior 5D field (x,y,k,l,m)
-  long long force_gen = 0;      // changes with every rt_set_forcing
+  long long args_gen = 0;       // changes with what a batch's launches carry by value: the forcing, dt, dzt(1)
   double dzt1 = 0.0;            // dzt(1), the bottom cell's spacing
   SplitFluxes fastv{};          // fast binary64 step: V of the right faces and face-0 planes (allocated on selection)
   double* psi_mem = nullptr;    // its slope rings
@@ -449,7 +449,7 @@ struct rt_batch {
   std::vector<rt_handle*> mem;
   std::vector<int> cur0;        // members' ping-pong index when the arrays were built
   std::vector<int> forced;      // members with a forcing, when the arrays were built
-  std::vector<long long> fgen;  // and every member's forcing generation then
+  std::vector<long long> gen;   // and every member's args_gen then
   int fp64 = 0;
   int parity = 0;               // steps taken since the arrays were built, mod 2
   cudaStream_t st = nullptr;
@@ -831,10 +831,10 @@ static int batch_build(rt_batch* b) {
   }
   b->parity = 0;
   b->forced.clear();
-  b->fgen.assign(b->mem.size(), 0);
+  b->gen.assign(b->mem.size(), 0);
   for (size_t j = 0; j < b->mem.size(); j++) {
     if (b->mem[j]->forcing != RT_FORCING_NONE) b->forced.push_back((int)j);
-    b->fgen[j] = b->mem[j]->force_gen;
+    b->gen[j] = b->mem[j]->args_gen;
   }
   // capture graph_steps launches starting at each parity
   batch_free_graphs(b);
@@ -855,13 +855,19 @@ static int batch_build(rt_batch* b) {
   return RT_OK;
 }
 
+// the arrays and graphs are stale once a member was stepped on its own, or
+// its forcing, dt or grid changed, since the build
+static void batch_look(rt_batch* b) {
+  const size_t n = b->mem.size();
+  for (size_t j = 0; j < n; j++)
+    if (b->mem[j]->cur != (b->cur0[j] ^ b->parity) || b->gen.size() != n || b->mem[j]->args_gen != b->gen[j])
+      b->dirty = true;
+}
+
 template <class T>
 static int batch_run(rt_batch* b, int nsteps) {
   const int n = (int)b->mem.size();
-  for (int j = 0; j < n; j++)  // a member stepped on its own, or its forcing changed, since the build
-    if (b->mem[j]->cur != (b->cur0[j] ^ b->parity) || b->fgen.size() != (size_t)n ||
-        b->mem[j]->force_gen != b->fgen[j])
-      b->dirty = true;
+  batch_look(b);
   // binary64 members: the batch kernels read uCFL, which a member's own fast
   // steps may have replaced (queued on the member's stream, ordered below)
   for (int j = 0; j < n; j++)
@@ -1023,8 +1029,8 @@ int rt_batch_dry(rt_batch* b, int nsteps) {
   for (int j = 0; j < n; j++) {
     BCUDA_TRY(b, cudaEventRecord(b->mem[j]->ev, b->mem[j]->st));
     BCUDA_TRY(b, cudaStreamWaitEvent(b->st, b->mem[j]->ev, 0));
-    if (b->mem[j]->cur != (b->cur0[j] ^ b->parity)) b->dirty = true;
   }
+  batch_look(b);
   if (b->dirty) {
     int rc = b->fp64 ? batch_build<double>(b) : batch_build<float>(b);
     if (rc) return rc;
@@ -1231,6 +1237,7 @@ int rt_set_grid(rt_handle* h, const double* dxt, const double* dyt, const double
     CUDA_TRY(h, cudaMemcpy(h->grid + h->goff[k], src[k], n * sizeof(double), cudaMemcpyHostToDevice));
   }
   h->dzt1 = dzt[pidx(1)];
+  h->args_gen += 1;
   h->uniform = 1;
   for (int a = 0; a < 6; a++)
     for (int f = 1; f <= h->d.n[a]; f++)   // faces 0..n
@@ -1258,6 +1265,7 @@ int rt_set_dt(rt_handle* h, double dt) {
   if (!h) return RT_ERR_ARG;
   if (!(dt > 0.0)) return fail(h, RT_ERR_ARG, "rt_set_dt: dt must be > 0");
   h->p.dt = dt;
+  h->args_gen += 1;
   if (h->have_grid) {
     int rc = upload_tab32(h);
     if (rc) return rc;
@@ -1482,7 +1490,7 @@ int rt_set_forcing(rt_handle* h, int kind, const double* F) {
   const long long nplane = (long long)d.n[0] * d.n[1] * d.nspec;
   // the work on the stream may still read the old field
   CUDA_TRY(h, cudaStreamSynchronize(h->st));
-  h->force_gen += 1;
+  h->args_gen += 1;
   h->forcing = RT_FORCING_NONE;
   if (kind == RT_FORCING_NONE) return RT_OK;
   if (!h->force) {
