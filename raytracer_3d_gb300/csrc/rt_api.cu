@@ -62,7 +62,7 @@ struct rt_handle {
   int slab_state = 0;           // 0: not asked for yet, 1: there, -1: no memory for it
   double* nu = nullptr;         // a cell's factor in the fast step (allocated on selection)
   double* tab64 = nullptr;      // and its tables 1/d_a (offsets toff[0..5])
-  int uc_holds = 0;             // uc/ucl hold 0: uCFL of the bit-exact kernels, 1: H of the fast step
+  int uc_holds = -1;            // uc/ucl hold 0: uCFL of the bit-exact kernels, 1: H of the fast step, -1: neither
   double* scratch = nullptr;    // reductions
   long long scratch_len = 0;
   double* coeff_mem = nullptr;  // small fields: scratch of rt_calc_parameter
@@ -1238,6 +1238,7 @@ int rt_set_grid(rt_handle* h, const double* dxt, const double* dyt, const double
   }
   h->dzt1 = dzt[pidx(1)];
   h->args_gen += 1;
+  h->uc_holds = -1;   // a budget before the next rt_calc_parameter must not read the old grid's uCFL
   h->uniform = 1;
   for (int a = 0; a < 6; a++)
     for (int f = 1; f <= h->d.n[a]; f++)   // faces 0..n
@@ -1266,6 +1267,7 @@ int rt_set_dt(rt_handle* h, double dt) {
   if (!(dt > 0.0)) return fail(h, RT_ERR_ARG, "rt_set_dt: dt must be > 0");
   h->p.dt = dt;
   h->args_gen += 1;
+  h->uc_holds = -1;
   if (h->have_grid) {
     int rc = upload_tab32(h);
     if (rc) return rc;
