@@ -139,6 +139,15 @@ static int tmp_alloc(rt_handle* h, void** ptr, size_t n) {
   return RT_OK;
 }
 
+// host array to device memory that queued work may read: in the handle's
+// stream, behind that work and ahead of what is queued next (a copy on the
+// default stream is ordered with neither).  The caller waits for the stream
+// before the host array goes.
+static int copy_in(rt_handle* h, void* dst, const void* src, size_t n) {
+  CUDA_TRY(h, cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, h->st));
+  return RT_OK;
+}
+
 static long long padded_len(const Dims& d, int a) { return d.n[a] + 2 * RT_ONX; }
 
 // ---------------------------------------------------------------------------
@@ -427,8 +436,9 @@ static int upload_tab32(rt_handle* h) {
       t[h->toff[12 + a] + i] = chi;
       t[h->toff[18 + a] + i] = (float)(c - (double)chi);
     }
-  CUDA_TRY(h, cudaMemcpy(h->tab32, t.data(), t.size() * sizeof(float), cudaMemcpyHostToDevice));
-  return RT_OK;
+  const int rc = copy_in(h, h->tab32, t.data(), t.size() * sizeof(float));
+  CUDA_TRY(h, cudaStreamSynchronize(h->st));
+  return rc;
 }
 
 // after a synchronisation: report a device-side wait that timed out
@@ -1228,14 +1238,15 @@ int rt_set_grid(rt_handle* h, const double* dxt, const double* dyt, const double
   const double* src[9] = {dxt, dyt, dzt, dkt, dlt, dmt, kt, lt, mt};
   for (int k = 0; k < 9; k++) {
     if (!src[k]) return fail(h, RT_ERR_ARG, "rt_set_grid: array %d is NULL", k);
-    const int a = k < 6 ? k : k - 3;
-    const long long n = padded_len(h->d, a);
-    if (k < 6)
-      for (long long i = 0; i < n; i++)
-        if (!(src[k][i] > 0.0))
-          return fail(h, RT_ERR_GRID, "rt_set_grid: spacing %d at padded index %lld is not > 0", k, i);
-    CUDA_TRY(h, cudaMemcpy(h->grid + h->goff[k], src[k], n * sizeof(double), cudaMemcpyHostToDevice));
+    for (long long i = 0; k < 6 && i < padded_len(h->d, k); i++)
+      if (!(src[k][i] > 0.0))
+        return fail(h, RT_ERR_GRID, "rt_set_grid: spacing %d at padded index %lld is not > 0", k, i);
   }
+  for (int k = 0; k < 9; k++) {
+    const int rc = copy_in(h, h->grid + h->goff[k], src[k], padded_len(h->d, k < 6 ? k : k - 3) * sizeof(double));
+    if (rc) return rc;
+  }
+  CUDA_TRY(h, cudaStreamSynchronize(h->st));
   h->dzt1 = dzt[pidx(1)];
   h->args_gen += 1;
   h->uc_holds = -1;   // a budget before the next rt_calc_parameter must not read the old grid's uCFL
@@ -1254,9 +1265,11 @@ int rt_set_background(rt_handle* h, const double* Nsqr, const double* U, const d
   if (!h) return RT_ERR_ARG;
   if (!Nsqr || !U || !V) return fail(h, RT_ERR_ARG, "rt_set_background: NULL array");
   const double* src[3] = {Nsqr, U, V};
-  for (int k = 0; k < 3; k++)
-    CUDA_TRY(h, cudaMemcpy(h->bg + k * h->bglen, src[k], h->bglen * sizeof(double),
-                           cudaMemcpyHostToDevice));
+  for (int k = 0; k < 3; k++) {
+    const int rc = copy_in(h, h->bg + k * h->bglen, src[k], h->bglen * sizeof(double));
+    if (rc) return rc;
+  }
+  CUDA_TRY(h, cudaStreamSynchronize(h->st));
   h->have_bg = true;
   h->have_coeff = false;
   return RT_OK;
@@ -1512,7 +1525,9 @@ int rt_set_forcing(rt_handle* h, int kind, const double* F) {
           std::memcpy(&f[(size_t)q], row, (size_t)d.n[0] * sizeof(double));
           q += d.n[0];
         }
-  CUDA_TRY(h, cudaMemcpy(h->force, f.data(), f.size() * sizeof(double), cudaMemcpyHostToDevice));
+  const int rc = copy_in(h, h->force, f.data(), f.size() * sizeof(double));
+  if (rc) return rc;
+  CUDA_TRY(h, cudaStreamSynchronize(h->st));
   h->forcing = kind;
   return RT_OK;
 }
