@@ -642,6 +642,14 @@ static cudaError_t batch_launch(rt_batch* b, int par, bool force = true) {
   return launch_batch<T>(mem, b->d_first, n, b->smem, b->tune.threads, b->grid, b->st);
 }
 
+// member arrays into the device memory that the batch's queued launches may
+// still read: in the batch's stream, behind them
+static cudaError_t batch_copy(rt_batch* b, void* dst, const void* src, size_t n) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, b->st);
+  const cudaError_t w = cudaStreamSynchronize(b->st);
+  return e != cudaSuccess ? e : w;
+}
+
 // binary32 members whose planes fill the fully staged kernel's CTA form the
 // persistent class; its arrays, stage size and grid
 template <class T>
@@ -687,11 +695,10 @@ static int batch_build_persistent(rt_batch* b, std::vector<int>& rest) {
   }
   for (int par = 0; par < 2; par++) {
     if (!b->d_pmem[par]) BCUDA_TRY(b, cudaMalloc(&b->d_pmem[par], (size_t)n * sizeof(BatchMember<float>)));
-    BCUDA_TRY(b, cudaMemcpy(b->d_pmem[par], arr[par].data(), pm.size() * sizeof(BatchMember<float>),
-                            cudaMemcpyHostToDevice));
+    BCUDA_TRY(b, batch_copy(b, b->d_pmem[par], arr[par].data(), pm.size() * sizeof(BatchMember<float>)));
   }
   if (!b->d_pfirst) BCUDA_TRY(b, cudaMalloc(&b->d_pfirst, (size_t)(n + 1) * sizeof(long long)));
-  BCUDA_TRY(b, cudaMemcpy(b->d_pfirst, first.data(), first.size() * sizeof(long long), cudaMemcpyHostToDevice));
+  BCUDA_TRY(b, batch_copy(b, b->d_pfirst, first.data(), first.size() * sizeof(long long)));
   const int per_sm = batch_w3_blocks_per_sm(b->pthreads, b->pR, batch_w3_smem(b->pns, b->pstage));
   if (per_sm < 1) return bfail(b, RT_ERR_CUDA, "batched staged kernel does not fit on an SM");
   int dev = 0, nsm = 0;
@@ -743,11 +750,10 @@ static int batch_build_slices(rt_batch* b, std::vector<int>& rest) {
   }
   for (int par = 0; par < 2; par++) {
     if (!b->d_smem6[par]) BCUDA_TRY(b, cudaMalloc(&b->d_smem6[par], (size_t)n * sizeof(BatchMember<float>)));
-    BCUDA_TRY(b, cudaMemcpy(b->d_smem6[par], arr[par].data(), sm.size() * sizeof(BatchMember<float>),
-                            cudaMemcpyHostToDevice));
+    BCUDA_TRY(b, batch_copy(b, b->d_smem6[par], arr[par].data(), sm.size() * sizeof(BatchMember<float>)));
   }
   if (!b->d_sfirst) BCUDA_TRY(b, cudaMalloc(&b->d_sfirst, (size_t)(n + 1) * sizeof(long long)));
-  BCUDA_TRY(b, cudaMemcpy(b->d_sfirst, first.data(), first.size() * sizeof(long long), cudaMemcpyHostToDevice));
+  BCUDA_TRY(b, batch_copy(b, b->d_sfirst, first.data(), first.size() * sizeof(long long)));
   const int per_sm = w6_blocks_per_sm(nt, w6_smem(ns, stage));
   if (per_sm < 1) return bfail(b, RT_ERR_CUDA, "batched z-slice kernel does not fit on an SM");
   int dev = 0, nsm = 0;
@@ -822,12 +828,10 @@ static int batch_build(rt_batch* b) {
     const int nall = (int)b->mem.size();
     for (int par = 0; par < 2; par++) {
       if (!b->d_mem[par]) BCUDA_TRY(b, cudaMalloc(&b->d_mem[par], (size_t)nall * sizeof(BatchMember<T>)));
-      BCUDA_TRY(b, cudaMemcpy(b->d_mem[par], arr[par].data(), (size_t)n * sizeof(BatchMember<T>),
-                              cudaMemcpyHostToDevice));
+      BCUDA_TRY(b, batch_copy(b, b->d_mem[par], arr[par].data(), (size_t)n * sizeof(BatchMember<T>)));
     }
     if (!b->d_first) BCUDA_TRY(b, cudaMalloc(&b->d_first, (size_t)(nall + 1) * sizeof(long long)));
-    BCUDA_TRY(b, cudaMemcpy(b->d_first, first.data(), (size_t)(n + 1) * sizeof(long long),
-                            cudaMemcpyHostToDevice));
+    BCUDA_TRY(b, batch_copy(b, b->d_first, first.data(), (size_t)(n + 1) * sizeof(long long)));
     b->smem = smem;
     b->tma = tma;
     b->group = group;
