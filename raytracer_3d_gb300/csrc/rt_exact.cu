@@ -421,13 +421,23 @@ long long exact_scratch_z0(const Dims& d) {
   return ax == 2 ? d.s[2] : exact_slab_planes(d) * (d.s[ax] / d.n[2]);
 }
 
+// cells per CTA: one CTA per SM, so that the binary64 work spreads evenly;
+// fewer where the face lists would outgrow the 48 KB of shared memory that a
+// launch may have without asking (GPUs of less than 139 SMs).  Asking is by an
+// attribute of the kernel that all handles and host threads share.
+int exact_small_cells(const Dims& d, int sms) {
+  int lists = 1;   // slots per cell: two per active axis, one for the z face 0
+  for (int a = 0; a < 6; a++) lists += d.n[a] > 1 ? 2 : 0;
+  const int most = (48 * 1024 - 64) / 8 / lists;
+  return (int)std::min<long long>(most, (d.ncell + sms - 1) / sms);
+}
+
 namespace {
 
-// cells per CTA: one CTA per SM, so that the binary64 work spreads evenly
-SmallGeom make_small(const Dims& d, int ctas) {
+SmallGeom make_small(const Dims& d, int sms) {
   SmallGeom S;
   S.G = make_cells(d);
-  S.C = (int)((d.ncell + ctas - 1) / ctas);
+  S.C = exact_small_cells(d, sms);
   S.axes = 0;
   int at = 0;
   for (int a = 0; a < 6; a++) {
@@ -470,13 +480,11 @@ cudaError_t launch_step_exact_small(const StepArgs<double>& A, int nsteps, int f
     if (jobs <= threads) kernel = exact_small_kernel<1, 2>;
     else if (jobs <= 2 * threads) kernel = exact_small_kernel<2, 2>;
   }
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  if (e != cudaSuccess) return e;
   if (nsteps == 1) {
     kernel<<<ctas, threads, sm, st>>>(A, S, W, 1, nullptr);
     return cudaGetLastError();
   }
-  e = cudaMemsetAsync(counter, 0, sizeof(unsigned), st);
+  cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned), st);
   if (e != cudaSuccess) return e;
   StepArgs<double> a = A;
   SmallGeom s = S;

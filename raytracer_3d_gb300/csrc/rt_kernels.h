@@ -176,6 +176,8 @@ bool exact_in_slabs(const Dims& d);
 // doubles of the slab scratch: flux field of axis a, and the face-0 plane of z
 long long exact_scratch(const Dims& d, int a);
 long long exact_scratch_z0(const Dims& d);
+// cells per CTA of the one-launch form on a GPU of `sms` multiprocessors
+int exact_small_cells(const Dims& d, int sms);
 cudaError_t launch_step_exact_small(const StepArgs<double>& A, int nsteps, int forcing, const double* F, double dz,
                                     unsigned* counter, cudaStream_t st);
 // energy budget of the step from A.E to Ecur by the same slabs: terms: scratch
