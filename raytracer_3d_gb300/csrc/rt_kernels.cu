@@ -478,16 +478,11 @@ template bool tma_path_ok<float>(const Dims&);
 template size_t tma_path_smem<double>(const Dims&);
 template size_t tma_path_smem<float>(const Dims&);
 
-template <class T, int NT, class K>
-static cudaError_t set_smem(K kernel, size_t bytes) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
 template <class T, int NT, int MAXC>
 static cudaError_t launch_tma_nt_c(const StepArgs<T>& A, const PlaneSched& S, long long nblk,
                                    cudaStream_t st) {
   const size_t sm = tma_smem<T>(A.d);
-  cudaError_t e = set_smem<T, NT>(step_tma_kernel<T, NT, MAXC>, sm);
+  cudaError_t e = set_smem(step_tma_kernel<T, NT, MAXC>, sm);
   if (e != cudaSuccess) return e;
   step_tma_kernel<T, NT, MAXC><<<(unsigned)nblk, NT, sm, st>>>(A, S);
   return cudaGetLastError();
@@ -506,7 +501,7 @@ template <class T, int NT>
 static cudaError_t launch_group_nt(const StepArgs<T>& A, const PlaneSched& S, long long nblk,
                                    cudaStream_t st) {
   const size_t sm = group_smem<T>(A.d, S.gz);
-  cudaError_t e = set_smem<T, NT>(step_group_kernel<T, NT>, sm);
+  cudaError_t e = set_smem(step_group_kernel<T, NT>, sm);
   if (e != cudaSuccess) return e;
   step_group_kernel<T, NT><<<(unsigned)nblk, NT, sm, st>>>(A, S);
   return cudaGetLastError();
@@ -585,14 +580,14 @@ static int occ_batch(bool tma, size_t smem, bool group = false) {
   int nb = 0;
   cudaError_t e;
   if (group) {
-    e = set_smem<T, NT>(batch_group_kernel<T, NT>, smem);
+    e = set_smem(batch_group_kernel<T, NT>, smem);
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, batch_group_kernel<T, NT>, NT, smem);
   } else if (tma) {
     // one MAXC for the occupancy query: register use differs little
-    e = set_smem<T, NT>(batch_tma_kernel<T, NT, 1>, smem);
-    if (e == cudaSuccess) e = set_smem<T, NT>(batch_tma_kernel<T, NT, 2>, smem);
-    if (e == cudaSuccess) e = set_smem<T, NT>(batch_tma_kernel<T, NT, 4>, smem);
+    e = set_smem(batch_tma_kernel<T, NT, 1>, smem);
+    if (e == cudaSuccess) e = set_smem(batch_tma_kernel<T, NT, 2>, smem);
+    if (e == cudaSuccess) e = set_smem(batch_tma_kernel<T, NT, 4>, smem);
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, batch_tma_kernel<T, NT, 4>, NT, smem);
   } else {

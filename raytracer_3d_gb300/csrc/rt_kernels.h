@@ -9,6 +9,22 @@ namespace rt {
 struct Phys;
 template <class T> struct StepArgs;
 
+// lets launches of `kernel` have `bytes` of dynamic shared memory.  The limit
+// belongs to the kernel, not to a launch: every handle, batch and host thread
+// shares it.  So it only goes up, to all that the device gives a CTA.
+template <class K>
+cudaError_t set_smem(K kernel, size_t bytes) {
+  cudaFuncAttributes a;
+  cudaError_t e = cudaFuncGetAttributes(&a, (const void*)kernel);
+  if (e != cudaSuccess || bytes <= (size_t)a.maxDynamicSharedSizeBytes) return e;
+  int dev = 0, most = 0;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+  if (bytes + a.sharedSizeBytes > (size_t)most) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              most - (int)a.sharedSizeBytes);
+}
+
 // binary32 literal 1e-12 of diagnose.f90:56, widened to binary64
 #define RT_LIT_1EM12 9.9999999600419720e-13
 

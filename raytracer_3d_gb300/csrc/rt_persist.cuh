@@ -17,11 +17,6 @@ namespace rt {
 
 inline int most_cells(long long nxy, int nt) { return (int)((nxy + nt - 1) / nt); }
 
-template <class K>
-cudaError_t set_smem(K kernel, size_t bytes) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
 inline int sm_count() {
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
