@@ -179,9 +179,10 @@ int rt_get_tendency(rt_handle* h, double* dE, double* meanfl);
  *   2  = the default.  binary64: the reference's arithmetic with its
  *        divisions on the integer pipes, one launch for small fields and two
  *        passes over slabs of the slowest axis for the others (the slab's
- *        flux fields are allocated by the first such step: 48 bytes per cell
- *        of a slab of about 2 M cells or one plane of the slowest axis; a
- *        handle without room for them steps with the plane kernel).
+ *        flux fields are allocated by rt_calc_parameter, or by this call
+ *        after it: 48 bytes per cell of a slab of about 2 M cells or one
+ *        plane of the slowest axis; a handle without room for them steps
+ *        with the plane kernel).
  *        binary32: threads marching along k, the next k's operands copied
  *        ahead into shared memory; fields above 2^30 cells: plane tiled with
  *        bulk-copy (TMA) staging of the E planes

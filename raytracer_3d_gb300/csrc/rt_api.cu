@@ -56,7 +56,7 @@ struct rt_handle {
   double* psi[7]{};             // by axis, and the reflected z face 0
   unsigned short* signs = nullptr;  // velocity signs per cell
   int uniform = 0;              // every axis has one spacing
-  SplitFluxes slab{};           // flux scratch of the bit-exact step's slabs (allocated by the first such step)
+  SplitFluxes slab{};           // flux scratch of the bit-exact step's slabs (allocated by the set-up)
   double* slab_mem = nullptr;
   double* terms = nullptr;      // terms of the budget's wavenumber integrals, one slab (allocated by the first budget)
   int slab_state = 0;           // 0: not asked for yet, 1: there, -1: no memory for it
@@ -311,7 +311,10 @@ static cudaError_t ensure_uc(rt_handle* h, int kind) {
 static bool fast_ready(const rt_handle* h) { return h->psi_mem && h->nu && h->tab64 && h->signs; }
 
 // scratch of the bit-exact step's slabs, one allocation; false when the
-// memory is not there (the handle then keeps the fused kernels, which need none)
+// memory is not there (the handle then keeps the fused kernels, which need
+// none).  Called by the set-up and by budgets, never by a step: a step may be
+// under capture, and must not wait for other streams.  Stream-ordered for
+// that reason too.
 static bool slab_scratch(rt_handle* h) {
   if (h->slab_state) return h->slab_state > 0;
   long long len[7], total = 0;
@@ -320,7 +323,7 @@ static bool slab_scratch(rt_handle* h) {
     total += (len[a] + 1) / 2 * 2;
   }
   double* p = nullptr;
-  if (cudaMalloc((void**)&p, (size_t)total * sizeof(double)) != cudaSuccess) {
+  if (cudaMallocAsync((void**)&p, (size_t)total * sizeof(double), h->st) != cudaSuccess) {
     cudaGetLastError();
     h->slab_state = -1;
     return false;
@@ -339,7 +342,7 @@ static bool slab_scratch(rt_handle* h) {
 static bool budget_scratch(rt_handle* h) {
   if (h->terms) return true;
   const size_t n = (size_t)budget_terms(h->d) * sizeof(double);
-  if (cudaMalloc((void**)&h->terms, n) != cudaSuccess) {
+  if (cudaMallocAsync((void**)&h->terms, n, h->st) != cudaSuccess) {
     cudaGetLastError();
     h->terms = nullptr;
     return false;
@@ -356,6 +359,14 @@ static bool exact_variant(const rt_handle* h) {
          v != RT_VARIANT_CELL && v != RT_VARIANT_GROUP && h->d.ncell < (1ll << 31);
 }
 
+// set-up: what the steps of this handle work with, asked for anew where there
+// was no memory the last time
+static void step_scratch(rt_handle* h) {
+  if (!h->have_coeff || !exact_variant(h) || !exact_in_slabs(h->d)) return;
+  if (h->slab_state < 0) h->slab_state = 0;
+  slab_scratch(h);
+}
+
 // one step of the handle from buffer src into 1 - src; returns the kernels launched
 static cudaError_t step_once(rt_handle* h, int src, int* nlaunch) {
   if (h->p.precision == RT_FP64) {
@@ -370,7 +381,7 @@ static cudaError_t step_once(rt_handle* h, int src, int* nlaunch) {
       *nlaunch = 1;
       if (!exact_in_slabs(h->d))
         return launch_step_exact_small(make_step_args<double>(h, src), 1, RT_FORCING_NONE, nullptr, 0.0, nullptr, h->st);
-      if (slab_scratch(h)) return launch_step_exact_slabs(make_step_args<double>(h, src), h->slab, h->st, nlaunch);
+      if (h->slab_state > 0) return launch_step_exact_slabs(make_step_args<double>(h, src), h->slab, h->st, nlaunch);
     }
     *nlaunch = 1;
     return launch_step<double>(make_step_args<double>(h, src), h->tune, h->st);
@@ -1335,6 +1346,7 @@ int rt_calc_parameter(rt_handle* h) {
   if (e == cudaSuccess) e = e2;
   if (e != cudaSuccess) return fail(h, RT_ERR_CUDA, "coefficients: %s", cudaGetErrorString(e));
   h->have_coeff = true;
+  step_scratch(h);
   return refresh_ucfl(h);
 }
 
@@ -1792,6 +1804,7 @@ int rt_set_tuning(rt_handle* h, int variant, int band, int threads) {
   h->tune.variant = variant;
   h->tune.band = band;
   h->tune.threads = threads;
+  step_scratch(h);
   return RT_OK;
 }
 
