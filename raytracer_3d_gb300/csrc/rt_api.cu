@@ -58,7 +58,9 @@ struct rt_handle {
   int uniform = 0;              // every axis has one spacing
   SplitFluxes slab{};           // flux scratch of the bit-exact step's slabs (allocated by the set-up)
   double* slab_mem = nullptr;
+  long long slab_bytes = 0;
   double* terms = nullptr;      // terms of the budget's wavenumber integrals, one slab (allocated by the first budget)
+  long long terms_bytes = 0;
   int slab_state = 0;           // 0: not asked for yet, 1: there, -1: no memory for it
   double* nu = nullptr;         // a cell's factor in the fast step (allocated on selection)
   double* tab64 = nullptr;      // and its tables 1/d_a (offsets toff[0..5])
@@ -114,8 +116,31 @@ static int fail(rt_handle* h, int code, const char* fmt, ...) {
                   __FILE__, __LINE__);                                                 \
   } while (0)
 
+// gives back the scratch that the handle works without where it has to
+// (slab_state, terms); false when it holds none
+static bool release_scratch(rt_handle* h) {
+  if (!h->slab_mem && !h->terms) return false;
+  cudaStreamSynchronize(h->st);   // queued steps may work with it
+  cudaFree(h->slab_mem);
+  cudaFree(h->terms);
+  h->bytes -= h->slab_bytes + h->terms_bytes;
+  h->slab_mem = h->terms = nullptr;
+  h->slab_bytes = h->terms_bytes = 0;
+  h->slab = SplitFluxes{};
+  h->slab_state = 0;
+  int dev = 0;
+  cudaMemPool_t pool;
+  if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
+    cudaMemPoolTrimTo(pool, 0);
+  return true;
+}
+
 static int dev_alloc(rt_handle* h, void** ptr, size_t n) {
   cudaError_t e = cudaMalloc(ptr, n);
+  if (e == cudaErrorMemoryAllocation && release_scratch(h)) {
+    cudaGetLastError();
+    e = cudaMalloc(ptr, n);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     *ptr = nullptr;
@@ -130,6 +155,10 @@ static int dev_alloc(rt_handle* h, void** ptr, size_t n) {
 // does not synchronise with work running on other streams (a batch)
 static int tmp_alloc(rt_handle* h, void** ptr, size_t n) {
   cudaError_t e = cudaMallocAsync(ptr, n, h->st);
+  if (e == cudaErrorMemoryAllocation && release_scratch(h)) {
+    cudaGetLastError();
+    e = cudaMallocAsync(ptr, n, h->st);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     *ptr = nullptr;
@@ -328,7 +357,8 @@ static bool slab_scratch(rt_handle* h) {
     h->slab_state = -1;
     return false;
   }
-  h->bytes += total * (long long)sizeof(double);
+  h->slab_bytes = total * (long long)sizeof(double);
+  h->bytes += h->slab_bytes;
   h->slab_mem = p;
   for (int a = 0; a < 7; a++) {
     (a < 6 ? h->slab.f[a] : h->slab.f0[2]) = len[a] > 0 ? p : nullptr;
@@ -347,7 +377,8 @@ static bool budget_scratch(rt_handle* h) {
     h->terms = nullptr;
     return false;
   }
-  h->bytes += (long long)n;
+  h->terms_bytes = (long long)n;
+  h->bytes += h->terms_bytes;
   return true;
 }
 
@@ -1720,6 +1751,7 @@ int rt_get_tendency(rt_handle* h, double* dE, double* meanfl) {
 cleanup:
   for (void* p : dev)
     if (p) cudaFreeAsync(p, h->st);
+  step_scratch(h);   // where it made room for the buffers
   return rc;
 }
 

@@ -1,5 +1,6 @@
 """Steps allocate nothing: what a handle works with is there once its
-coefficients and schedule are, so the first step can be captured."""
+coefficients and schedule are, so the first step can be captured.  Scratch
+that a handle can do without makes room for what a call cannot."""
 import numpy as np
 import pytest
 
@@ -58,4 +59,32 @@ def test_first_step_under_capture(precision, schedule, n, steps):
         graph.replay()
     m.sync()
     assert np.array_equal(m.get_state(), want)
+    m.close()
+
+
+def test_scratch_makes_room():
+    """rt_get_tendency beside a full GPU: its two fields fit only where the
+    scratch of the steps and budgets was; later steps have theirs again"""
+    import __graft_entry__ as g
+    g.build()
+    torch = pytest.importorskip("torch")
+    n = (32, 32, 32, 8, 8, 16)
+    m = configs.build_model(configs.shear_mini(n=n), "fp64")
+    m.integrate(2)
+    m.diagnose(fields=False)
+    want = m.get_tendency()
+    m.sync()
+    held = m.device_bytes()
+    need = 2 * 8 * 32 ** 3 * 1024
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    filler = torch.empty(free - need + (40 << 20), dtype=torch.uint8, device="cuda")
+    got = m.get_tendency()
+    assert all(np.array_equal(x, y) for x, y in zip(got, want))
+    del filler
+    torch.cuda.empty_cache()
+    assert m.device_bytes() >= held - 16 * 2 ** 22      # all but the budget's
+    m.integrate(1)
+    b, _ = m.diagnose(fields=False)
+    assert m.device_bytes() == held and np.isfinite(b["residual"])
     m.close()
