@@ -328,6 +328,14 @@ int rt_fp64_rate(double* fma_per_s);
  * wait completed, 0 expected).  It touches no handle. */
 int rt_selftest_wait_timeout(int* status, int* completed);
 
+/* Self-test of the kernels that stand in where a handle's usual ones cannot
+ * run: on = 1 lets it (and a batch that it is a member of) work as if its
+ * optional scratch had found no memory and its field were beyond the binary32
+ * march, on = 0 (the state of a new handle) as ever.  Binary64 steps and the
+ * budget give the same bits either way (the budget's scalar sums to rounding),
+ * binary32 steps too.  No use in production. */
+int rt_selftest_fallback(rt_handle* h, int on);
+
 #ifdef __cplusplus
 }
 #endif

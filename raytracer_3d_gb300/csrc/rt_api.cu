@@ -61,6 +61,7 @@ struct rt_handle {
   long long slab_bytes = 0;
   double* terms = nullptr;      // terms of the budget's wavenumber integrals, one slab (allocated by the first budget)
   long long terms_bytes = 0;
+  bool fallback = false;        // rt_selftest_fallback
   int slab_state = 0;           // 0: not asked for yet, 1: there, -1: no memory for it
   double* nu = nullptr;         // a cell's factor in the fast step (allocated on selection)
   double* tab64 = nullptr;      // and its tables 1/d_a (offsets toff[0..5])
@@ -345,6 +346,7 @@ static bool fast_ready(const rt_handle* h) { return h->psi_mem && h->nu && h->ta
 // under capture, and must not wait for other streams.  Stream-ordered for
 // that reason too.
 static bool slab_scratch(rt_handle* h) {
+  if (h->fallback) return false;
   if (h->slab_state) return h->slab_state > 0;
   long long len[7], total = 0;
   for (int a = 0; a < 7; a++) {
@@ -823,7 +825,7 @@ static int batch_build(rt_batch* b) {
   const int n = (int)qm.size();
   b->nq = n;
   bool march = sizeof(T) == 4 && n > 0;
-  for (int j : qm) march = march && march_ok(b->mem[j]->d);
+  for (int j : qm) march = march && march_ok(b->mem[j]->d) && !b->mem[j]->fallback;
   for (int par = 0; par < 2; par++) {
     b->march[par].clear();
     if (march)
@@ -1837,6 +1839,17 @@ int rt_set_tuning(rt_handle* h, int variant, int band, int threads) {
   h->tune.band = band;
   h->tune.threads = threads;
   step_scratch(h);
+  return RT_OK;
+}
+
+int rt_selftest_fallback(rt_handle* h, int on) {
+  if (!h) return RT_ERR_ARG;
+  if (on != 0 && on != 1) return fail(h, RT_ERR_ARG, "rt_selftest_fallback: on must be 0 or 1");
+  h->fallback = on != 0;
+  h->tune.march = on == 0;
+  h->args_gen += 1;   // a batch picks its kernels anew
+  if (h->fallback) release_scratch(h);
+  else step_scratch(h);
   return RT_OK;
 }
 

@@ -515,7 +515,8 @@ cudaError_t launch_step(const StepArgs<T>& A, const StepTuning& tn, cudaStream_t
     // the z march, 30x18x20x14x10x12 54 against 33, 8x32x8x12x16x8 87 against 22
     // for z slices, 15x9x21x8x16x10 44 against 13 for one thread per cell)
     const int v = tn.variant;
-    if ((v == RT_VARIANT_TMA || v == RT_VARIANT_W2Q || v == RT_VARIANT_SPLIT || v == RT_VARIANT_FAST) && march_ok(A.d))
+    if ((v == RT_VARIANT_TMA || v == RT_VARIANT_W2Q || v == RT_VARIANT_SPLIT || v == RT_VARIANT_FAST) &&
+        tn.march && march_ok(A.d))
       return launch_march(A, tn, st);
     bool done = false;
     cudaError_t e = launch_persist(A, tn, st, done);

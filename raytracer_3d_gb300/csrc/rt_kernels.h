@@ -96,6 +96,7 @@ struct StepTuning {
   int threads = 512;  // CTA size of the plane kernels (128, 256, 512)
   int sweep = 0;      // 0: bands over m, 1: bands over l
   int group = 0;      // z planes per item of the group kernel (0: from the CTA size)
+  bool march = true;  // false: as if the field were beyond the k march (rt_selftest_fallback)
 };
 struct PlaneSched;
 PlaneSched make_sched(const Dims& d, const StepTuning& tn);
