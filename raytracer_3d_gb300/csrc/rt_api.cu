@@ -1351,13 +1351,16 @@ int rt_calc_parameter(rt_handle* h) {
   const Grid g = make_grid(h);
 
   // scratch of the dispersion relation: a ring of m planes, 256 MB or the
-  // three planes it cannot do without.  A small one stays with the handle
+  // three planes it cannot do without (a binary64 field beside which not even
+  // those fit takes the direct evaluation).  A small one stays with the handle
   // (taking 1.4 MB from the stream-ordered pool and giving it back cost 0.3 ms)
   double* scratch = nullptr;
   int ring = coeff_ring(d, 256ll << 20);
   const bool small = coeff_scratch(d, ring) * (long long)sizeof(double) <= (16ll << 20);
   int rc = RT_OK;
-  if (small) {
+  if (h->fallback && h->p.precision == RT_FP64) {
+    rc = RT_ERR_NOMEM;
+  } else if (small) {
     if (!h->coeff_mem) rc = dev_alloc(h, (void**)&h->coeff_mem, (size_t)coeff_scratch(d, ring) * sizeof(double));
     scratch = h->coeff_mem;
   } else {
@@ -1367,14 +1370,15 @@ int rt_calc_parameter(rt_handle* h) {
       rc = tmp_alloc(h, (void**)&scratch, (size_t)coeff_scratch(d, ring) * sizeof(double));
     }
   }
-  if (rc) return rc;
+  const bool fp64 = h->p.precision == RT_FP64, direct = rc == RT_ERR_NOMEM && fp64;
+  if (rc && !direct) return rc;
   int nl = 0;
-  cudaError_t e = h->p.precision == RT_FP64
-                      ? launch_coeff(d, bg, g, ph, coeff_out<double>(h), scratch, ring, h->result, &nl, h->st)
-                      : launch_coeff(d, bg, g, ph, coeff_out<float>(h), scratch, ring, h->result, &nl, h->st);
+  cudaError_t e = direct ? launch_coeff_direct(d, bg, g, ph, coeff_out<double>(h), h->result, &nl, h->st)
+                  : fp64 ? launch_coeff(d, bg, g, ph, coeff_out<double>(h), scratch, ring, h->result, &nl, h->st)
+                         : launch_coeff(d, bg, g, ph, coeff_out<float>(h), scratch, ring, h->result, &nl, h->st);
   h->launches += nl;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&h->rate, h->result, sizeof(double), cudaMemcpyDeviceToHost, h->st);
-  if (!small) cudaFreeAsync(scratch, h->st);   // stream-ordered: after the kernels
+  if (!small && scratch) cudaFreeAsync(scratch, h->st);   // stream-ordered: after the kernels
   const cudaError_t e2 = cudaStreamSynchronize(h->st);
   if (e == cudaSuccess) e = e2;
   if (e != cudaSuccess) return fail(h, RT_ERR_CUDA, "coefficients: %s", cudaGetErrorString(e));

@@ -62,6 +62,9 @@ long long coeff_scratch(const Dims& d, int ring);
 template <class T>
 cudaError_t launch_coeff(const Dims& d, const Background& bg, const Grid& g, const Phys& ph, const CoeffOut<T>& out,
                          double* scratch, int ring, double* rate, int* nlaunch, cudaStream_t st);
+// the same of a binary64 field without scratch (rt_coeff_direct.cu)
+cudaError_t launch_coeff_direct(const Dims& d, const Background& bg, const Grid& g, const Phys& ph,
+                                const CoeffOut<double>& out, double* rate, int* nlaunch, cudaStream_t st);
 // padded host array (pageable, read / written by the GPU directly) <-> the
 // unpadded device field; the scatter also writes *status to the host int *hstatus
 template <class T>

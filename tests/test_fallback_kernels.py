@@ -1,6 +1,7 @@
 """The kernels that stand in where the usual ones cannot run (no memory for the
-exact step's slabs and the budget's terms; binary32 fields beyond the march),
-on small fields: the same bits as the one-thread-per-cell kernel."""
+exact step's slabs and the budget's terms, or for the dispersion relation of
+the coefficients; binary32 fields beyond the march), on small fields: the same
+bits as the one-thread-per-cell kernel, and as the usual coefficients."""
 import numpy as np
 import pytest
 
@@ -106,3 +107,30 @@ def test_batch_beyond_the_march(shapes):
     b.close()
     for m in models:
         m.close()
+
+
+@pytest.mark.parametrize("walls", [True, False])
+@pytest.mark.parametrize("n", [
+    (6, 5, 6, 4, 4, 6), (16, 3, 7, 8, 2, 10), (5, 4, 3, 2, 1, 2), (1, 6, 8, 4, 6, 4), (9, 1, 6, 6, 4, 2),
+    (1, 1, 12, 1, 1, 20), (40, 30, 1, 1, 1, 1),
+])
+def test_coefficients_without_scratch(n, walls):
+    import __graft_entry__ as g
+    g.build()
+    m = _model(n, "fp64", walls, False)
+    fields = [m.get_field(w) for w in range(9)]
+    rate = m.max_rate()
+    m.integrate(3)
+    E = m.get_state()
+    m.set_state()
+    m._check(m._lib.rt_selftest_fallback(m.handle, 1), "rt_selftest_fallback")
+    m.U *= 2.0                       # other coefficients first, so that nothing is left from before
+    m.calc_parameter()
+    m.U *= 0.5
+    m.calc_parameter()
+    assert m.max_rate() == rate
+    for w, want in enumerate(fields):
+        assert np.array_equal(m.get_field(w), want), w
+    m.integrate(3)
+    assert np.array_equal(m.get_state(), E)
+    m.close()
