@@ -202,7 +202,7 @@ int rt_get_tendency(rt_handle* h, double* dE, double* meanfl);
  *        per cell and rings of slopes, 1.3 GB at 32^6 cells);
  *        within a few units in the last place of the reference's result per
  *        step, NOT bit-identical to it.  band and threads have no effect;
- *        fields of 2^31 cells or more are rejected (RT_ERR_CUDA on the step)
+ *        fields of 2^31 cells or more are rejected (RT_ERR_ARG)
  * Every other variant gives the same result: bit-identical to the
  * reference's arithmetic in binary64, and among themselves in binary32.
  * band: values per band of the plane schedule (default 8); threads: CTA

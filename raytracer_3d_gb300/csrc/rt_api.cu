@@ -1836,6 +1836,7 @@ int rt_set_tuning(rt_handle* h, int variant, int band, int threads) {
   if (threads != 128 && threads != 256 && threads != 512 && threads != 1024)
     return fail(h, RT_ERR_ARG, "rt_set_tuning: threads must be 128, 256, 512 or 1024");
   if (variant == RT_VARIANT_FAST && h->p.precision == RT_FP64) {
+    if (!fast_ok(h->d)) return fail(h, RT_ERR_ARG, "rt_set_tuning: the fast step takes fields below 2^31 cells");
     const int rc = ensure_fast(h);
     if (rc) return rc;
   }

@@ -286,8 +286,13 @@ long long fast_ring(const Dims& d, int a) {
   return r;
 }
 
+// the kernels index cells with 32 bits
+bool fast_ok(const Dims& d) { return d.ncell < (1ll << 31); }
+
 cudaError_t launch_fast_prepare(const Dims& d, const Grid& g, double dt, const FastFields& C, double* tab,
                                 const long long* toff, int* nlaunch, cudaStream_t st) {
+  *nlaunch = 0;
+  if (!fast_ok(d)) return cudaErrorInvalidValue;
   *nlaunch = 2;
   fast_prepare_kernel<<<8 * 152, 256, 0, st>>>(d, g, dt, C, make_cells(d));
   cudaError_t e = cudaGetLastError();
@@ -299,7 +304,7 @@ cudaError_t launch_fast_prepare(const Dims& d, const Grid& g, double dt, const F
 cudaError_t launch_step_fast(const Dims& d, const FastFields& C, const double* E, double* Enew, int* nlaunch,
                              cudaStream_t st) {
   *nlaunch = 0;
-  if (d.ncell >= (1ll << 31)) return cudaErrorInvalidValue;
+  if (!fast_ok(d)) return cudaErrorInvalidValue;
   const CellGeom G = make_cells(d);
   const long long slab = slab_cells(d);
   const bool xw = d.n[0] >= 2 && 32 % d.n[0] == 0;

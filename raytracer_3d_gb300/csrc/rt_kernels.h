@@ -229,6 +229,7 @@ struct FastFields {
   const double* inv_d[6];
   int uniform;
 };
+bool fast_ok(const Dims& d);   // fields below 2^31 cells
 long long fast_ring(const Dims& d, int a);
 cudaError_t launch_fast_prepare(const Dims& d, const Grid& g, double dt, const FastFields& C, double* tab,
                                 const long long* toff, int* nlaunch, cudaStream_t st);
