@@ -89,6 +89,11 @@ typedef struct {
  * (parallel_mpi.f90:16-25: nk, nl, nm even or one). */
 int rt_create(const rt_dims* dims, const rt_params* params, rt_handle** out);
 int rt_destroy(rt_handle* h);
+/* Device memory of a handle of these sizes, without creating it: *resident
+ * from rt_calc_parameter on (rt_device_bytes then, with the default schedule
+ * and neither forcing nor budgets), *transient the scratch that
+ * rt_calc_parameter takes and gives back.  Needs no GPU. */
+int rt_footprint(const rt_dims* dims, const rt_params* params, long long* resident, long long* transient);
 /* message of the last error on h (or of the last failed rt_create for NULL) */
 const char* rt_last_error(const rt_handle* h);
 

@@ -47,6 +47,8 @@ _P = ctypes.c_void_p
 _D = ctypes.POINTER(ctypes.c_double)
 SIGNATURES = {
     "rt_create": (ctypes.c_int, [ctypes.POINTER(RtDims), ctypes.POINTER(RtParams), ctypes.POINTER(_P)]),
+    "rt_footprint": (ctypes.c_int, [ctypes.POINTER(RtDims), ctypes.POINTER(RtParams),
+                                    ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong)]),
     "rt_destroy": (ctypes.c_int, [_P]),
     "rt_last_error": (ctypes.c_char_p, [_P]),
     "rt_set_grid": (ctypes.c_int, [_P] + [_D] * 9),

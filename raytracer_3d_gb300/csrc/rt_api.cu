@@ -178,6 +178,10 @@ static int copy_in(rt_handle* h, void* dst, const void* src, size_t n) {
   return RT_OK;
 }
 
+// scratch of rt_calc_parameter: what its ring may take, and up to what size it
+// stays with the handle
+constexpr long long kCoeffRing = 256ll << 20, kCoeffKept = 16ll << 20;
+
 static long long padded_len(const Dims& d, int a) { return d.n[a] + 2 * RT_ONX; }
 
 // ---------------------------------------------------------------------------
@@ -340,6 +344,18 @@ static cudaError_t ensure_uc(rt_handle* h, int kind) {
 
 static bool fast_ready(const rt_handle* h) { return h->psi_mem && h->nu && h->tab64 && h->signs; }
 
+// length of the slabs' scratch, and of its parts: flux fields by axis, the z
+// face-0 plane
+static long long slab_doubles(const Dims& d, long long len[7]) {
+  long long total = 0;
+  for (int a = 0; a < 7; a++) {
+    const long long n = a < 6 ? exact_scratch(d, a) : exact_scratch_z0(d);
+    if (len) len[a] = n;
+    total += (n + 1) / 2 * 2;
+  }
+  return total;
+}
+
 // scratch of the bit-exact step's slabs, one allocation; false when the
 // memory is not there (the handle then keeps the fused kernels, which need
 // none).  Called by the set-up and by budgets, never by a step: a step may be
@@ -348,11 +364,8 @@ static bool fast_ready(const rt_handle* h) { return h->psi_mem && h->nu && h->ta
 static bool slab_scratch(rt_handle* h) {
   if (h->fallback) return false;
   if (h->slab_state) return h->slab_state > 0;
-  long long len[7], total = 0;
-  for (int a = 0; a < 7; a++) {
-    len[a] = a < 6 ? exact_scratch(h->d, a) : exact_scratch_z0(h->d);
-    total += (len[a] + 1) / 2 * 2;
-  }
+  long long len[7];
+  const long long total = slab_doubles(h->d, len);
   double* p = nullptr;
   if (cudaMallocAsync((void**)&p, (size_t)total * sizeof(double), h->st) != cudaSuccess) {
     cudaGetLastError();
@@ -1148,6 +1161,50 @@ const char* rt_version(void) { return "raytracer_gb300 0.1 (sm_103a)"; }
 
 const char* rt_last_error(const rt_handle* h) { return h ? h->err.c_str() : g_create_err.c_str(); }
 
+static void fill_dims(Dims& d, const int nn[6], const rt_params* params) {
+  long long st = 1;
+  for (int a = 0; a < 6; a++) {
+    d.n[a] = nn[a];
+    d.s[a] = st;
+    st *= nn[a];
+  }
+  d.ncell = st;
+  d.nvol3 = (long long)nn[0] * nn[1] * nn[2];
+  d.nspec = (long long)nn[3] * nn[4] * nn[5];
+  d.upper_refl = params->enable_upper_reflection ? 1 : 0;
+  d.lower_refl = params->enable_lower_reflection ? 1 : 0;
+  fill_plane_strides(d);
+}
+
+// what rt_create and rt_calc_parameter allocate, summed (held against
+// rt_device_bytes in the tests)
+int rt_footprint(const rt_dims* dims, const rt_params* params, long long* resident, long long* transient) {
+  if (!dims || !params || !resident || !transient) return fail(nullptr, RT_ERR_ARG, "rt_footprint: NULL argument");
+  const int nn[6] = {dims->nx, dims->ny, dims->nz, dims->nk, dims->nl, dims->nm};
+  for (int a = 0; a < 6; a++)
+    if (nn[a] < 1) return fail(nullptr, RT_ERR_ARG, "rt_footprint: axis %d has %d points", a, nn[a]);
+  if (params->precision != RT_FP64 && params->precision != RT_FP32)
+    return fail(nullptr, RT_ERR_ARG, "rt_footprint: unknown precision %d", params->precision);
+  Dims d{};
+  fill_dims(d, nn, params);
+  const bool fp64 = params->precision == RT_FP64;
+  long long planes = 0, line = 0, tables = 0;
+  for (int a = 0; a < 6; a++) {
+    planes += d.ncell / d.n[a];
+    line += padded_len(d, a) * (a < 3 ? 1 : 2);   // spacings, and the wavenumbers of k, l, m
+    tables += 4 * padded_len(d, a);
+  }
+  long long n = (fp64 ? 8 : 4) * ((2 + 6 + (fp64 ? 3 : 1)) * d.ncell + planes);   // E, velocities, growth rates
+  if (fp64) n += 8 * (6 * d.ncell + planes);                                      // uCFL
+  n += 8 * line + 4 * tables + 3 * 8 * padded_len(d, 0) * padded_len(d, 1) * padded_len(d, 2);
+  n += 8 * (diag_sizes(d).scratch_doubles() + 8) + 8 * 8 * d.nvol3 + 32 * 8 + 2 * sizeof(int) + 2 * sizeof(unsigned);
+  if (fp64 && d.ncell < (1ll << 31) && exact_in_slabs(d)) n += 8 * slab_doubles(d, nullptr);
+  const long long coeff = 8 * coeff_scratch(d, coeff_ring(d, kCoeffRing));
+  *resident = n + (coeff <= kCoeffKept ? coeff : 0);
+  *transient = coeff <= kCoeffKept ? 0 : coeff;
+  return RT_OK;
+}
+
 int rt_create(const rt_dims* dims, const rt_params* params, rt_handle** out) {
   if (!dims || !params || !out) return fail(nullptr, RT_ERR_ARG, "rt_create: NULL argument");
   *out = nullptr;
@@ -1178,19 +1235,8 @@ int rt_create(const rt_dims* dims, const rt_params* params, rt_handle** out) {
 
   rt_handle* h = new rt_handle();
   h->p = *params;
-  Dims& d = h->d;
-  long long st = 1;
-  for (int a = 0; a < 6; a++) {
-    d.n[a] = nn[a];
-    d.s[a] = st;
-    st *= nn[a];
-  }
-  d.ncell = st;
-  d.nvol3 = (long long)nn[0] * nn[1] * nn[2];
-  d.nspec = (long long)nn[3] * nn[4] * nn[5];
-  d.upper_refl = params->enable_upper_reflection ? 1 : 0;
-  d.lower_refl = params->enable_lower_reflection ? 1 : 0;
-  fill_plane_strides(d);
+  fill_dims(h->d, nn, params);
+  const Dims& d = h->d;
   h->elem = params->precision == RT_FP64 ? 8 : 4;
 
   auto bail = [&](int code) {
@@ -1355,8 +1401,8 @@ int rt_calc_parameter(rt_handle* h) {
   // those fit takes the direct evaluation).  A small one stays with the handle
   // (taking 1.4 MB from the stream-ordered pool and giving it back cost 0.3 ms)
   double* scratch = nullptr;
-  int ring = coeff_ring(d, 256ll << 20);
-  const bool small = coeff_scratch(d, ring) * (long long)sizeof(double) <= (16ll << 20);
+  int ring = coeff_ring(d, kCoeffRing);
+  const bool small = coeff_scratch(d, ring) * (long long)sizeof(double) <= kCoeffKept;
   int rc = RT_OK;
   if (h->fallback && h->p.precision == RT_FP64) {
     rc = RT_ERR_NOMEM;

@@ -5,9 +5,9 @@ A request is one wave-field integration (an `Experiment` plus a step
 count).  The loop:
 
   1. admits arrived requests in arrival order while their device footprint
-     (resident fields plus the transient binary64 coefficient buffers of the
-     set-up) fits the budget; set-up of a new member runs on its own stream
-     while the current batch chunk runs on the batch stream;
+     (what the member holds plus the scratch of its set-up) fits the budget;
+     set-up of a new member runs on its own stream while the current batch
+     chunk runs on the batch stream;
   2. advances every active member by one chunk of steps with one batched,
      graph-captured launch per step (chunk = min(chunk_max, fewest steps any
      member has left), so every member stops exactly at its step count);
@@ -18,6 +18,7 @@ Latency of a request = completion time - arrival time.  The executor is
 pluggable so the scheduling logic is testable without a GPU
 (`FakeExecutor`).
 """
+import ctypes
 import math
 import time
 from dataclasses import dataclass, field
@@ -66,13 +67,23 @@ def poisson_requests(n, rate, seed, steps_range=(50, 1000), spatial=None, spectr
     return out
 
 
+def member_bytes(n, precision):
+    """(resident, transient) device bytes of a member of extents n: what it
+    holds once set up, and the scratch of the dispersion relation that its
+    set-up gives back (rt_footprint)"""
+    from . import _lib
+    dims = _lib.RtDims(*n, 2)
+    par = _lib.RtParams(1.0, 1e-4, 1.0, 1, 1, _lib.RT_FP64 if precision == "fp64" else _lib.RT_FP32)
+    res, tmp = ctypes.c_longlong(), ctypes.c_longlong()
+    _lib.check(_lib.load().rt_footprint(ctypes.byref(dims), ctypes.byref(par), ctypes.byref(res), ctypes.byref(tmp)),
+               None, "rt_footprint")
+    return res.value, tmp.value
+
+
 def bytes_per_cell(precision):
-    """resident device bytes per cell and transient set-up bytes per cell"""
-    elem = 8 if precision == "fp64" else 4
-    nlam = 3 if precision == "fp64" else 1
-    resident = elem * (2 + 6 + nlam) + elem * 6 / 8.0      # + face-0 planes (<= n/8 of a field)
-    transient = 0 if precision == "fp64" else 8 * (6 + 3) + 8 * 6 / 8.0
-    return resident, transient
+    """member_bytes per cell of a small member (4 points per axis), whose
+    fixed parts and kept scratch weigh more than those of larger ones"""
+    return tuple(b / 4.0 ** 6 for b in member_bytes((4,) * 6, precision))
 
 
 @dataclass
@@ -281,8 +292,7 @@ class GpuExecutor:
             time.sleep(d)
 
     def footprint(self, r):
-        res, tmp = bytes_per_cell(self.precision)
-        return res * r.cells, tmp * r.cells
+        return member_bytes(r.exp.n, self.precision)
 
     def admit(self, r):
         from .configs import build_model
