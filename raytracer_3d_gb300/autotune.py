@@ -67,13 +67,20 @@ def _event_timer(stream_ptr):
     return timed
 
 
+# Kinds of cache entries.  A number goes up when the names in a kind's entries
+# come to mean other kernels: an older choice was timed against those that are
+# gone.  (model2, batch5: 'tma', 'split' and 'w2q' are the march and the exact
+# step over slabs, a batch without classes is the march.)
+MODEL_KIND, BATCH_KIND = "model2", "batch5"
+
+
 def signature(kind, shapes, precision):
     return "%s|%s|%s" % (kind, precision, ";".join("x".join(map(str, s)) for s in shapes))
 
 
 def tune_model(model, candidates=None, reps=3, use_cache=True):
     """Pick the fastest schedule for one Model; returns (best, table)."""
-    key = signature("model", [model.n], model.precision)
+    key = signature(MODEL_KIND, [model.n], model.precision)
     cache = _load_cache() if use_cache else {}
     if use_cache and key in cache:
         best = tuple(cache[key]["best"])
@@ -115,7 +122,7 @@ def tune_batch(batch, candidates=None, reps=2, graph_steps=16, use_cache=True):
     the consumer threads of the two staged classes (0: off) and whether
     they share one launch for a Batch; returns (best, table) with best =
     (band, threads, sweep, persistent, slices, fused)."""
-    key = signature("batch4", sorted(m.n for m in batch.models), batch.models[0].precision)
+    key = signature(BATCH_KIND, sorted(m.n for m in batch.models), batch.models[0].precision)
     cache = _load_cache() if use_cache else {}
 
     def apply(c):
