@@ -382,10 +382,13 @@ constexpr long long kSlabCells = 1ll << 21;
 // slabs side by side in one launch, as the fast step has them: 7.84 ms, and
 // three slabs of scratch.)
 constexpr unsigned kReadyBlocks = 1024;
-// Largest field stepped in one launch, both faces of every axis per cell
-// (twice the flux work, one launch less): 160x300 took 10.3 us against 14.4
-// in two passes, 6x6x8x6^3 (62,208 cells) 24.8 against 24.5, 10x20x24x24
-// (115,200) 26.7 against 22.6.
+// Largest field stepped in one launch.  us per step in one launch / in two
+// passes, as single steps and, behind the comma, in a run of 200: 160x300
+// 10.3 / 12.3, 8.0 / 12.3; 64x1024 12.3 / 12.3, 9.0 / 12.3; 6x6x8x6^3 (62,208
+// cells) 24.0 / 20.5, 21.1 / 22.5; 4^3x8^2x16 (65,536) 24.6 / 21.3, 21.6 / 22.5;
+// 100x1000 16.4 / 14.4, 13.5 / 14.4.  Just beyond the line a CTA's lists of a 6D
+// field no longer fit 48 KB, the CTAs take two rounds, and 4^3x8^2x20 (81,920)
+// measures 45 / 24.6, 45 / 26.7.
 constexpr long long kOneLaunchCells = 1ll << 16;
 
 int slab_axis(const Dims& d) {

@@ -164,7 +164,7 @@ __host__ __device__ __forceinline__ double sqrt_rn(double x) {
   const int E = expo(b) - 1023;
   const uint64_t m = significand(b) << (E & 1);               // x = m/2^52 * 4^(E >> 1), m/2^52 in [1, 4)
   // reciprocal root of the first 24 bits, lowered by eight units in the last
-  // place (the instruction is within two): below the true one by less than 2^-19.8
+  // place (the instruction is within two): below the true one by less than 2^-19.7
   const uint32_t fb = (127u << 23) + ((E & 1) ? (1u << 23) : 0u) + ((b.hi & 0xfffffu) << 3) + (b.lo >> 29);
   float f, r;
 #ifdef __CUDA_ARCH__

@@ -84,13 +84,13 @@ cudaError_t launch_ucfl(const Dims& d, const Grid& g, double dt, const double* c
 // binary32 kernels that were measured slower and removed.
 #define RT_VARIANT_PLANE 0
 #define RT_VARIANT_CELL 1
-#define RT_VARIANT_TMA 2
+#define RT_VARIANT_TMA 2      // the default: rt_exact.cu, rt_march.cu; the TMA planes where those cannot run
 #define RT_VARIANT_GROUP 3
 #define RT_VARIANT_W3 9       // binary32: every operand staged by TMA
 #define RT_VARIANT_W6 13      // binary32: small planes, z slices per item
 #define RT_VARIANT_W2Z 14     // binary32: 2-wide blocks, z-march
-#define RT_VARIANT_W2Q 18     // the same with the cell-pair arithmetic on packed f32x2 instructions and
-                              // the next plane's operands prefetched into L2 (the binary32 production step)
+#define RT_VARIANT_W2Q 18     // binary32: as TMA up to 2^30 cells; above, W2Z with the cell-pair arithmetic on packed
+                              // f32x2 instructions and the next plane's operands prefetched into L2
 #define RT_VARIANT_SPLIT 15   // binary64: every face flux once, two passes (rt_exact.cu)
 #define RT_VARIANT_FAST 16    // binary64: without divisions, slopes on the integer pipes (rt_fast.cu), within 1e-12 of the reference
 struct StepTuning {

@@ -2,8 +2,8 @@
 // the dispatch over every persistent variant (launch_persist), the form with
 // every operand staged by TMA (rt_step8.cuh, RT_VARIANT_W3) single-field and
 // batched, and the small-plane form with z slices per item (rt_step11.cuh,
-// RT_VARIANT_W6, also the ensemble class of small planes).  The production
-// 2-wide z-march kernel is instantiated in rt_persist_w2.cu so the library
+// RT_VARIANT_W6, also the ensemble class of small planes).  The 2-wide z-march
+// kernel is instantiated in rt_persist_w2.cu so the library
 // builds in parallel.
 #include "rt_persist.cuh"
 

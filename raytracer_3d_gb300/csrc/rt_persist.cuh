@@ -5,7 +5,7 @@
 //                     (rt_step8.cuh, RT_VARIANT_W3) single-field and batched,
 //                     the small-plane z-slice kernel (rt_step11.cuh,
 //                     RT_VARIANT_W6) single-field and batched;
-//   rt_persist_w2.cu  the production 2-wide block kernel marching along z
+//   rt_persist_w2.cu  the 2-wide block kernel marching along z
 //                     (rt_step7.cuh, RT_VARIANT_W2Z).
 #pragma once
 #include <algorithm>

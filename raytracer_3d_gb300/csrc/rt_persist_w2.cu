@@ -1,7 +1,8 @@
-// rt_persist_w2.cu -- launcher of the production binary32 step kernel
+// rt_persist_w2.cu -- launcher of the staged binary32 z-march kernel
 // (rt_step7.cuh: 2-wide blocks, CTAs marching along z over the (k,l,m)
-// columns; RT_VARIANT_W2Q with packed pair arithmetic and L2 prefetch of
-// the next plane, RT_VARIANT_W2Z the scalar form without prefetch).
+// columns; RT_VARIANT_W2Q, where it comes to that, with packed pair
+// arithmetic and L2 prefetch of the next plane, RT_VARIANT_W2Z the scalar form
+// without prefetch).
 #include "rt_persist.cuh"
 
 namespace rt {

@@ -1,4 +1,4 @@
-// rt_step2.cuh -- plane-tiled fused step (the production step kernel).
+// rt_step2.cuh -- plane-tiled fused step.
 //
 // One CTA updates one "plane": all nx*ny cells of one (z, k) pair at one
 // (l, m).  The plane of E is staged in shared memory, the x and y face

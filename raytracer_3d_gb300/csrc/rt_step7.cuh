@@ -1,4 +1,4 @@
-// rt_step7.cuh -- the production binary32 step: warp-specialised, multi-stage,
+// rt_step7.cuh -- the staged binary32 z march: warp-specialised, multi-stage,
 // 2-wide cell blocks, CTAs marching along z.
 //
 // Producer, stage ring and descriptors are those of rt_step6.cuh; each CTA
