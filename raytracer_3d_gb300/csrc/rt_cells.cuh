@@ -51,8 +51,7 @@ __device__ __forceinline__ int plane32(const CellGeom& G, int a, const int c[6])
   return q;
 }
 
-// face 0 of an axis whose lower ghosts copy the edge cell: Rj = 0 and the
-// flux is v*(E0+E0)*0.5 = v*E0 exactly
+// face 0 of an axis whose lower ghosts copy the edge cell: no limited slope
 __device__ __forceinline__ bool face0_is_copy(const Dims& d, int a) { return a != 2 || !d.lower_refl; }
 
 }  // namespace rt

@@ -199,7 +199,7 @@ __device__ __forceinline__ void cell_run(const StepArgs<double>& A, const SmallG
 #pragma unroll
   for (int f = 0; f < AX; f++) {
     if (f >= S.axes) break;
-    const double fl = J.left[f] >= 0 ? sF[J.left[f]] : dmul(J.v0[f], e0);
+    const double fl = J.left[f] >= 0 ? sF[J.left[f]] : face0_flux(J.v0[f], e0);
     q[f] = div_rn(dsub(sF[J.right[f]], fl), J.dd[f]);
   }
   double dE = 0.;
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(256, 8) exact_update_kernel(StepArgs<double> A
       fl = F.f[a][a == L.ax ? ring_at(L, p - L.s_ax, ca - 1) : q - G.s[a]];
     } else {
       const int q0 = plane32(G, a, c);
-      fl = face0_is_copy(d, a) ? dmul(A.vlo[a][q0], e0) : F.f0[a][q0 - L.q0];
+      fl = face0_is_copy(d, a) ? face0_flux(A.vlo[a][q0], e0) : F.f0[a][q0 - L.q0];
     }
     const double quo = div_rn(dsub(fr, fl), A.g.d[a][pidx(ca + 1)]);
     dE = first ? zero_minus(quo) : dsub(dE, quo);
@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(256, 3) budget_cells_kernel(StepArgs<double> A
         fl = F.f[a][a == L.ax ? ring_at(L, p - L.s_ax, ca - 1) : q - G.s[a]];
       } else {
         const int q0 = plane32(G, a, c);
-        fl = face0_is_copy(d, a) ? dmul(A.vlo[a][q0], e0) : F.f0[a][q0 - L.q0];
+        fl = face0_is_copy(d, a) ? face0_flux(A.vlo[a][q0], e0) : F.f0[a][q0 - L.q0];
       }
       dE = dsub(dE, div_rn(dsub(fr, fl), w[a]));
     }
@@ -640,7 +640,7 @@ __device__ __forceinline__ double face_at(const StepArgs<double>& A, const Split
                                           const Slab& L, bool hi, int p, const int c[6]) {
   if (hi) return F.f[a][a == L.ax ? ring_at(L, p, c[a]) : p - (int)L.base];
   const int q0 = plane32(G, a, c);
-  return face0_is_copy(A.d, a) ? dmul(A.vlo[a][q0], A.E[p]) : F.f0[a][q0 - L.q0];
+  return face0_is_copy(A.d, a) ? face0_flux(A.vlo[a][q0], A.E[p]) : F.f0[a][q0 - L.q0];
 }
 
 // a thread's share of the boundary sum through face 0 / n of axis a

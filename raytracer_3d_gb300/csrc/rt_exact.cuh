@@ -292,6 +292,17 @@ __device__ __forceinline__ double flux_exact(double v, double u, double Ea, doub
   return flux_of(v, u, S, Rj, limited_ratio(up, Rj));
 }
 
+// face 0 of an axis whose lower ghosts copy the edge cell: the reference's
+// (v*(E0+E0))*0.5 less a diffusive part of Rj = E0-E0, which is v*E0 in
+// mid_range (no sum or product overflows, none is denormal)
+__device__ __noinline__ static double face0_slow(double v, double e0) {
+  return dsub(dmul(dmul(v, dadd(e0, e0)), 0.5), dsub(e0, e0));
+}
+__device__ __forceinline__ double face0_flux(double v, double e0) {
+  if (!(mid_range(split64(v)) && mid_range(split64(e0)))) return face0_slow(v, e0);
+  return dmul(v, e0);
+}
+
 // ---- the flux with its differences on the integer pipes ----
 // Where the three E values a face's limiter depends on (its sides b and c,
 // and w behind the upwind side) lie within 2^8 of each other, they are
