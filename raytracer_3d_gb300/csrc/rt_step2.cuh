@@ -18,6 +18,7 @@
 // for bit; binary32: division-free limiter).  The divergence is accumulated
 // in the reference's axis order x, y, z, k, l, m.
 #pragma once
+#include "rt_exact.cuh"
 #include "rt_step.cuh"
 
 namespace rt {
@@ -27,11 +28,12 @@ template <class T> __device__ __forceinline__ void st_stream(T* p, T v) { __stcs
 
 // flux of face 0 of an open axis: the ghost cells copy cell 0, so
 // Rj = E(0)-E(-1) = 0 and the superbee diffusive term vanishes; the flux is
-// v*(E0+E0)*0.5 = v*E0 exactly (also in binary64, where the scaling by 2
-// and 0.5 is exact and a zero sign cannot change a later nonzero sum).
+// v*(E0+E0)*0.5 = v*E0 (binary64: exactly, but for overflows and denormals,
+// which face0_flux sends through the sequence; a zero's sign cannot change a
+// later nonzero sum).
 template <class T> __device__ __forceinline__ T open_face0_flux(T v, T e0);
 template <> __device__ __forceinline__ double open_face0_flux<double>(double v, double e0) {
-  return dmul(v, e0);
+  return face0_flux(v, e0);
 }
 template <> __device__ __forceinline__ float open_face0_flux<float>(float v, float e0) {
   return v * e0;

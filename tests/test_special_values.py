@@ -23,13 +23,14 @@ def _state(n, dtype, kinds, seed):
     return np.asfortranarray(E)
 
 
-def _run(n, precision, walls, E, variant, steps):
+def _run(n, precision, walls, E, variant, steps, fallback=0):
     exp = configs.shear_mini(n=n, upper=walls, lower=walls)
     exp.fixed = (1e-3, 0.0, 1e-2)
     m = configs.build_model(exp, precision, padded=False)
     m.E = E
     m.set_state()
     m.set_tuning(variant, 8, 256)
+    m._check(m._lib.rt_selftest_fallback(m.handle, fallback), "rt_selftest_fallback")
     for k in steps:
         m.integrate(k)
     out = m.get_state()
@@ -52,3 +53,26 @@ def test_special_values_equal_the_cell_kernel(precision, n, kinds):
         for steps in ((4,), (1, 1, 1, 1)):
             got = _run(n, precision, walls, E, "tma", steps)
             assert np.array_equal(got, want, equal_nan=True), (walls, steps)
+
+
+@pytest.mark.parametrize("kinds", [("denormal", "zero"), ("negative", "zero", "huge"), ("inf",), ("nan",)])
+@pytest.mark.parametrize("n", [(16, 8, 8, 6, 4, 6), (15, 7, 12, 4, 4, 6)])
+def test_special_values_in_the_plane_kernels(n, kinds):
+    import __graft_entry__ as g
+    g.build()
+    from raytracer_3d_gb300.batch import Batch
+    E = _state(n, np.float64, kinds, 9)
+    want = _run(n, "fp64", False, E, "cell", (3,))
+    for variant, fallback in (("plane", 0), ("group", 0), ("tma", 1)):
+        assert np.array_equal(_run(n, "fp64", False, E, variant, (3,), fallback), want, equal_nan=True), variant
+    exp = configs.shear_mini(n=n, upper=False, lower=False)
+    exp.fixed = (1e-3, 0.0, 1e-2)
+    m = configs.build_model(exp, "fp64", padded=False)
+    m.E = E
+    m.set_state()
+    b = Batch([m])
+    b.integrate(3)
+    b.sync()
+    assert np.array_equal(m.get_state(), want, equal_nan=True)
+    b.close()
+    m.close()
