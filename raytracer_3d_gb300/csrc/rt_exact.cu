@@ -14,12 +14,13 @@
 // The bound is the binary64 pipe: 7 instructions per face flux (10 where
 // values next to each other differ by more than 2^8), two per axis in the
 // divergence and seven in the update, 61 per cell with six axes in the two
-// passes (290 with the divisions on that pipe).  32x32x32x12^3 measured 7.57
-// ms per step, 7.5 G cells/s and 456 G binary64 instructions/s, 86% of the
-// measured rate (9.45 ms with 10 per flux); the TMA plane kernel took 39.9
-// ms, and a CTA of 512 threads per x-y plane 280 us for a 40x120 column
-// (one launch here: 8.2 us), 6.3 ms for a 10x20x60x60 section (79 us) and
-// 8.7 ms for 8x8x16x16^3 (0.58 ms).  The integer work (340 instructions per
+// passes (290 with the divisions on that pipe).  32x32x32x12^3 measures 7.22
+// ms per step, 7.8 G cells/s and 484 G binary64 instructions/s, 91% of the
+// measured rate (7.57 ms with the edge fluxes as bare multiplications in a
+// branch; 9.45 ms with 10 per flux); the TMA plane kernel took
+// 39.9 ms, and a CTA of 512 threads per x-y plane 280 us for a 40x120 column
+// (one launch here: 8.2 us), 6.3 ms for a 10x20x60x60 section (76 us) and
+// 8.7 ms for 8x8x16x16^3 (0.56 ms).  The integer work (340 instructions per
 // flux) wants many warps to hide behind: 32 registers and 8 resident CTAs
 // with some spilling measured 7.65 ms then, 40 and 6 CTAs 7.90, 48 and 5 CTAs
 // 8.15, 52 and 4 CTAs 8.40.
