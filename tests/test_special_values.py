@@ -76,3 +76,24 @@ def test_special_values_in_the_plane_kernels(n, kinds):
     assert np.array_equal(m.get_state(), want, equal_nan=True)
     b.close()
     m.close()
+
+
+@pytest.mark.parametrize("kinds", [("denormal", "zero"), ("negative", "zero", "huge")])
+@pytest.mark.parametrize("n", [(6, 5, 6, 4, 4, 6), (3, 4, 5, 10, 2, 6), (1, 1, 12, 1, 1, 20)])
+def test_edge_integrals_of_special_values(n, kinds):
+    """the budget's wavenumber integrals, edge fluxes among them, against the kernels that need no scratch"""
+    import __graft_entry__ as g
+    g.build()
+    got = []
+    for fallback in (0, 1):
+        exp = configs.shear_mini(n=n, upper=False, lower=False)
+        exp.fixed = (1e-3, 0.0, 1e-2)
+        m = configs.build_model(exp, "fp64", padded=False)
+        m._check(m._lib.rt_selftest_fallback(m.handle, fallback), "rt_selftest_fallback")
+        m.E = _state(n, np.float64, kinds, 10)
+        m.set_state()
+        m.integrate(1)
+        got.append(m.diagnose()[1])
+        m.close()
+    for k in got[0]:
+        assert np.array_equal(got[0][k], got[1][k], equal_nan=True), k
