@@ -63,6 +63,7 @@ struct rt_handle {
   long long terms_bytes = 0;
   bool fallback = false;        // rt_selftest_fallback
   int slab_state = 0;           // 0: not asked for yet, 1: there, -1: no memory for it
+  bool slab_kept = false;       // a captured step holds its address: it stays as long as the handle
   double* nu = nullptr;         // a cell's factor in the fast step (allocated on selection)
   double* tab64 = nullptr;      // and its tables 1/d_a (offsets toff[0..5])
   int uc_holds = -1;            // uc/ucl hold 0: uCFL of the bit-exact kernels, 1: H of the fast step, -1: neither
@@ -120,15 +121,21 @@ static int fail(rt_handle* h, int code, const char* fmt, ...) {
 // gives back the scratch that the handle works without where it has to
 // (slab_state, terms); false when it holds none
 static bool release_scratch(rt_handle* h) {
-  if (!h->slab_mem && !h->terms) return false;
+  const bool slab = h->slab_mem && !h->slab_kept;
+  if (!slab && !h->terms) return false;
   cudaStreamSynchronize(h->st);   // queued steps may work with it
-  cudaFree(h->slab_mem);
+  if (slab) {
+    cudaFree(h->slab_mem);
+    h->bytes -= h->slab_bytes;
+    h->slab_mem = nullptr;
+    h->slab_bytes = 0;
+    h->slab = SplitFluxes{};
+    h->slab_state = 0;
+  }
   cudaFree(h->terms);
-  h->bytes -= h->slab_bytes + h->terms_bytes;
-  h->slab_mem = h->terms = nullptr;
-  h->slab_bytes = h->terms_bytes = 0;
-  h->slab = SplitFluxes{};
-  h->slab_state = 0;
+  h->bytes -= h->terms_bytes;
+  h->terms = nullptr;
+  h->terms_bytes = 0;
   int dev = 0;
   cudaMemPool_t pool;
   if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
@@ -427,7 +434,15 @@ static cudaError_t step_once(rt_handle* h, int src, int* nlaunch) {
       *nlaunch = 1;
       if (!exact_in_slabs(h->d))
         return launch_step_exact_small(make_step_args<double>(h, src), 1, RT_FORCING_NONE, nullptr, 0.0, nullptr, h->st);
-      if (h->slab_state > 0) return launch_step_exact_slabs(make_step_args<double>(h, src), h->slab, h->st, nlaunch);
+      if (h->slab_state > 0 && !h->fallback) {
+        if (!h->slab_kept) {
+          cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+          const cudaError_t ec = cudaStreamIsCapturing(h->st, &cap);
+          if (ec != cudaSuccess) return ec;
+          h->slab_kept = cap != cudaStreamCaptureStatusNone;
+        }
+        return launch_step_exact_slabs(make_step_args<double>(h, src), h->slab, h->st, nlaunch);
+      }
     }
     *nlaunch = 1;
     return launch_step<double>(make_step_args<double>(h, src), h->tune, h->st);

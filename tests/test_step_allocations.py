@@ -88,3 +88,44 @@ def test_scratch_makes_room():
     b, _ = m.diagnose(fields=False)
     assert m.device_bytes() == held and np.isfinite(b["residual"])
     m.close()
+
+
+def test_scratch_of_a_captured_step_stays():
+    """a captured step holds the scratch's address: no call may give that
+    scratch away while the graph can still be launched"""
+    import __graft_entry__ as g
+    g.build()
+    torch = pytest.importorskip("torch")
+    from raytracer_3d_gb300._lib import RtError
+    n = (32, 32, 32, 8, 8, 16)
+    ref = _model(n, "fp64")
+    ref.integrate(6)
+    want = ref.get_state()
+    ref.close()
+    m = _model(n, "fp64")
+    m.sync()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(torch.cuda.ExternalStream(m.stream())):
+        graph.capture_begin(capture_error_mode="global")
+        try:
+            m.integrate(2)
+        finally:
+            graph.capture_end()
+        graph.replay()
+    m.integrate(2)
+    m.sync()
+    held = m.device_bytes()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    need = 2 * 8 * 32 ** 3 * 1024
+    filler = torch.empty(free - need + (40 << 20), dtype=torch.uint8, device="cuda")
+    with pytest.raises(RtError):
+        m.get_tendency()
+    assert m.device_bytes() == held
+    del filler
+    torch.cuda.empty_cache()
+    with torch.cuda.stream(torch.cuda.ExternalStream(m.stream())):
+        graph.replay()
+    m.sync()
+    assert np.array_equal(m.get_state(), want)
+    m.close()
