@@ -453,9 +453,11 @@ static cudaError_t step_once(rt_handle* h, int src, int* nlaunch) {
 
 // fast binary64 step: V for the axes with n > 1, the slope rings, nu, the
 // signs and the tables; a field with no such axis keeps the bit-exact step,
-// and so does one the step rejects
+// and so does one the step rejects.  Where they do not all fit, none is kept
 static int ensure_fast(rt_handle* h) {
+  if (fast_ready(h)) return RT_OK;
   const Dims& d = h->d;
+  const long long held = h->bytes - h->slab_bytes - h->terms_bytes;
   int rc = RT_OK;
   long long ring = 0;
   for (int a = 0; a < 6 && !rc; a++) {
@@ -478,6 +480,21 @@ static int ensure_fast(rt_handle* h) {
   if (!rc && !h->nu) rc = dev_alloc(h, (void**)&h->nu, (size_t)d.ncell * sizeof(double));
   if (!rc && !h->signs) rc = dev_alloc(h, (void**)&h->signs, (size_t)d.ncell * sizeof(unsigned short));
   if (!rc && !h->tab64) rc = dev_alloc(h, (void**)&h->tab64, (size_t)h->toff[6] * sizeof(double));
+  if (rc) {
+    for (int a = 0; a < 6; a++) {
+      cudaFree(h->fastv.f[a]);
+      cudaFree(h->fastv.f0[a]);
+      h->fastv.f[a] = h->fastv.f0[a] = nullptr;
+    }
+    cudaFree(h->psi_mem);
+    cudaFree(h->nu);
+    cudaFree(h->signs);
+    cudaFree(h->tab64);
+    h->psi_mem = h->nu = h->tab64 = nullptr;
+    h->signs = nullptr;
+    h->bytes = held + h->slab_bytes + h->terms_bytes;
+    step_scratch(h);   // where it made room for them
+  }
   return rc;
 }
 

@@ -129,3 +129,34 @@ def test_scratch_of_a_captured_step_stays():
     m.sync()
     assert np.array_equal(m.get_state(), want)
     m.close()
+
+
+def test_fast_that_does_not_fit_leaves_all_as_it_was():
+    """the fast step's fields on a full GPU: selection fails, and the handle
+    holds what it held, the step's scratch included"""
+    import __graft_entry__ as g
+    g.build()
+    torch = pytest.importorskip("torch")
+    from raytracer_3d_gb300._lib import RtError
+    n = (32, 32, 32, 8, 8, 16)
+    ref = _model(n, "fp64")
+    ref.integrate(3)
+    want = ref.get_state()
+    ref.close()
+    m = _model(n, "fp64")
+    m.integrate(1)
+    m.sync()
+    held = m.device_bytes()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    filler = torch.empty(free - (700 << 20), dtype=torch.uint8, device="cuda")    # two of its eight fields fit
+    with pytest.raises(RtError):
+        m.set_tuning("fast", 8, 256)
+    assert m.device_bytes() == held
+    m.integrate(2)
+    assert np.array_equal(m.get_state(), want)
+    del filler
+    torch.cuda.empty_cache()
+    m.set_tuning("fast", 8, 256)
+    assert m.device_bytes() > held
+    m.close()
