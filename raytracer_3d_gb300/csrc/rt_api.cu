@@ -618,7 +618,7 @@ static void batch_free_graphs(rt_batch* b) {
 // kernel launches per batch step
 static int batch_kernels(const rt_batch* b) {
   const int persistent = b->fgrid > 0 ? 1 : (b->np > 0 ? 1 : 0) + (b->ns6 > 0 ? 1 : 0);
-  const int rest = b->nq == 0 ? 0 : (b->march[0].empty() ? 1 : march_batch_launches(b->nq));
+  const int rest = b->nq == 0 ? 0 : (b->march[0].empty() ? 1 : march_batch_launches(b->march[0].data(), b->nq));
   return (int)b->forced.size() + persistent + rest;
 }
 

@@ -178,8 +178,10 @@ cudaError_t launch_persist(const StepArgs<float>& A, const StepTuning& tn, cudaS
 // to 2^30 cells
 bool march_ok(const Dims& d);
 cudaError_t launch_march(const StepArgs<float>& A, const StepTuning& tn, cudaStream_t st);
-// one step of n fields, in march_batch_launches(n) launches
-int march_batch_launches(int n);
+// one step of n fields, in march_batch_launches(S, n) launches, the first of
+// which takes march_batch_take(S, n) of them
+int march_batch_take(const StepArgs<float>* S, int n);
+int march_batch_launches(const StepArgs<float>* S, int n);
 cudaError_t launch_march_batch(const StepArgs<float>* A, int n, int band, int sweep, cudaStream_t st);
 // bit-exact binary64 step without binary64 divisions (rt_exact.cu).  Flux
 // fields of a two-pass step: f[a] (the cell's right face) and f0[a] (the

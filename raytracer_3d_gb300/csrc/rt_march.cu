@@ -114,14 +114,34 @@ cudaError_t launch_march(const StepArgs<float>& S, const StepTuning& tn, cudaStr
   return go(march_kernel<1>, 1, A.items, A, st);
 }
 
-int march_batch_launches(int n) { return (n + RT_MARCH_MEMBERS - 1) / RT_MARCH_MEMBERS; }
+// of n fields, those that one launch takes: what its arguments hold, and no
+// more CTAs than a grid may have (2^31 - 1; fields of one spatial point have a
+// CTA per (l,m), so two of 2^30 cells are beyond it)
+int march_batch_take(const StepArgs<float>* S, int n) {
+  long long ctas = 0;
+  int m = 0;
+  for (; m < std::min(n, RT_MARCH_MEMBERS); m++) {
+    const Dims& d = S[m].d;
+    const long long nvec = d.nvol3 / march_width(d);
+    // an upper bound of MarchArgs::items
+    ctas += (long long)d.n[4] * d.n[5] * ((nvec + RT_MARCH_THREADS - 1) / RT_MARCH_THREADS) + kBusy;
+    if (m > 0 && ctas > 0x7fffffffll) break;
+  }
+  return m;
+}
+
+int march_batch_launches(const StepArgs<float>* S, int n) {
+  int k = 0;
+  for (int j = 0; j < n; j += march_batch_take(S + j, n - j)) k++;
+  return k;
+}
 
 cudaError_t launch_march_batch(const StepArgs<float>* S, int n, int band, int sweep, cudaStream_t st) {
   long long cells = 0;
   for (int j = 0; j < n; j++) cells += S[j].d.ncell;
-  for (int j0 = 0; j0 < n; j0 += RT_MARCH_MEMBERS) {
+  for (int j0 = 0, take; j0 < n; j0 += take) {
     MarchBatch B;
-    B.nmem = std::min(n - j0, RT_MARCH_MEMBERS);
+    B.nmem = take = march_batch_take(S + j0, n - j0);
     unsigned total = 0;
     int V = 0;
     for (int j = 0; j < B.nmem; j++) {
