@@ -196,12 +196,27 @@ __device__ __forceinline__ void cell_run(const StepArgs<double>& A, const SmallG
   if (!J.live) return;
   const Dims& d = A.d;
   const double e0 = __ldcg(E + J.p);
-  double q[AX];   // the axes' quotients do not depend on one another
+  double fl[AX], q[AX];   // the axes' quotients do not depend on one another
+  bool easy = mid_range(split64(e0));
 #pragma unroll
   for (int f = 0; f < AX; f++) {
     if (f >= S.axes) break;
-    const double fl = J.left[f] >= 0 ? sF[J.left[f]] : face0_flux(J.v0[f], e0);
-    q[f] = div_rn(dsub(sF[J.right[f]], fl), J.dd[f]);
+    fl[f] = J.left[f] >= 0 ? sF[J.left[f]] : dmul(J.v0[f], e0);
+    easy = easy && mid_range(split64(J.v0[f]));
+  }
+  if (!easy) {   // one branch to face0_flux's slow path, ahead of the quotients, for one
+                 // per axis among them: 40x120 columns 188 -> 186 us per 50 steps, a host
+                 // step of 7x5x6x4x4x4 36.3 -> 35.4 us
+#pragma unroll
+    for (int f = 0; f < AX; f++) {
+      if (f >= S.axes) break;
+      if (J.left[f] < 0) fl[f] = face0_flux(J.v0[f], e0);
+    }
+  }
+#pragma unroll
+  for (int f = 0; f < AX; f++) {
+    if (f >= S.axes) break;
+    q[f] = div_rn(dsub(sF[J.right[f]], fl[f]), J.dd[f]);
   }
   double dE = 0.;
 #pragma unroll
